@@ -175,10 +175,10 @@ int Batch::launch_step(int step)
             BCU(launch_cg_stage_batch_mix(FB1, FB2, FB3, descm_[step & 1][irk], items_, (int)s.size(), work_,
                                           grid_ctas_, stream));
         else if (tile_ == 8)
-            BCU(ty8::launch_cg_stage_batch(FB1, FB2, FB3, desc_[irk], items_, (int)s.size(), work_, grid_ctas_,
+            BCU(ty8::launch_cg_stage_batch(FB1, FB2, FB3, irk, desc_[irk], items_, (int)s.size(), work_, grid_ctas_,
                                            stream));
         else
-            BCU(launch_cg_stage_batch(FB1, FB2, FB3, desc_[irk], items_, (int)s.size(), work_, grid_ctas_, stream));
+            BCU(launch_cg_stage_batch(FB1, FB2, FB3, irk, desc_[irk], items_, (int)s.size(), work_, grid_ctas_, stream));
         FB1 = -FB1, FB2 = -FB2, FB3 = -FB3;
     }
     for (Session *x : s)

@@ -1,0 +1,3 @@
+// The split pipeline of the CGFDM stage kernel on 32 x 4 tiles.
+#define CG_STAGE_SET 1
+#include "cgfdm_stage.cu"

@@ -1,0 +1,3 @@
+// The split pipeline of the CGFDM stage kernel on 32 x 8 tiles.
+#define CG_STAGE_SET 1
+#include "cgfdm_stage_ty8.cu"

@@ -113,15 +113,15 @@ struct CgStageArgs {
 struct CgStageMaps {
     alignas(64) unsigned char winp[128];   // the stencil input, point box (split pipeline)
     alignas(64) unsigned char win[128];
-    alignas(64) unsigned char cjm[128];
+    alignas(64) unsigned char cjm[128], cjm1[128];   // metric and medium: boxes of 3 fields and of 1 field
     alignas(64) unsigned char wm[128];
     alignas(64) unsigned char t[128];
 };
-// Everything one stage launch needs for one session: the four tensor maps
+// Everything one stage launch needs for one session: the tensor maps
 // (CUtensorMap, 128 bytes each, 64-byte aligned) and the arguments.
 // work: the launch's work-counter pair, zero between launches.
 struct alignas(64) CgStageDesc {
-    unsigned char tmW[128], tmC[128], tmM[128], tmT[128];
+    unsigned char tmW[128], tmC[128], tmC1[128], tmM[128], tmT[128];
     unsigned char tmS[128];   // mixed storage: the FP16 stencil-input delta, halo box
     unsigned char tmWc[128];  // split pipeline: the stencil input, interior column box
     CgStageArgs a;
@@ -144,12 +144,14 @@ struct alignas(64) CgStageDesc {
 // into out[0], out[1] (float bits; the caller sets out[0] to +inf bits and
 // out[1] to 0 first).  make_field_tmap: the 4-D tensor map (x, y, z, field)
 // of an nf-field buffer, with a halo box (40 x (tile rows + 4) x 1 x nf) or a
-// point box (32 x tile rows x 1 x nf); out must hold 128 bytes.
+// point box (32 x tile rows x 1 x nf), box_nf fields a box instead of nf
+// when given; out must hold 128 bytes.
 #define CG_STAGE_FUNCTIONS                                                                                         \
     cudaError_t launch_cg_stage(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,      \
                                 cudaStream_t st, bool halo_out = false);                                         \
-    cudaError_t launch_cg_stage_batch(int FB1, int FB2, int FB3, const CgStageDesc *descs, const int *item_start, \
-                                      int nsess, int *work, int grid_ctas, cudaStream_t st);                     \
+    cudaError_t launch_cg_stage_batch(int FB1, int FB2, int FB3, int irk, const CgStageDesc *descs,               \
+                                      const int *item_start, int nsess, int *work, int grid_ctas,                 \
+                                      cudaStream_t st);                                                          \
     size_t cg_stage_smem_bytes(bool mix = false);                                                               \
     size_t cg_stage2_smem_bytes();                                                                              \
     cudaError_t launch_cg_stage_split(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,\
@@ -162,8 +164,10 @@ struct alignas(64) CgStageDesc {
     int cg_stage_mix_ctas_per_sm();                                                                             \
     cudaError_t make_field_tmap16(void *out, const __half *base, const DevGrid &gh, int nf);                    \
     cudaError_t launch_impedance_bounds(const float *cjm, DevGrid g, unsigned *out, cudaStream_t st);           \
-    cudaError_t make_field_tmap(void *out, const float *base, const DevGrid &g, int nf, bool halo_box);         \
+    cudaError_t make_field_tmap(void *out, const float *base, const DevGrid &g, int nf, bool halo_box,          \
+                                int box_nf = 0);                                                                  \
     int cg_stage_ctas_per_sm();                                                                                 \
+    int cg_stage_split_ctas_per_sm();                                                                           \
     int cg_stage_tile_y();
 inline namespace ty4 {
 CG_STAGE_FUNCTIONS

@@ -565,6 +565,7 @@ void Session::stage_desc(int irk, CgStageDesc &d) const
     for (int f = 0; f < 6; f++) a.ho[f] = ho_[irk][f];
     std::memcpy(d.tmW, maps_[win_map[irk]].win, 128);
     std::memcpy(d.tmC, maps_[win_map[irk]].cjm, 128);
+    std::memcpy(d.tmC1, maps_[win_map[irk]].cjm1, 128);
     std::memcpy(d.tmM, maps_[win_map[irk]].wm, 128);
     std::memcpy(d.tmT, maps_[win_map[irk]].t, 128);
     std::memcpy(d.tmWc, maps_[win_map[irk]].winp, 128);
@@ -582,18 +583,23 @@ int Session::pml_faces() const
 
 int Session::stage_ctas_per_sm() const
 {
-    return mix_ ? cg_stage_mix_ctas_per_sm() : tile_ == 8 ? ty8::cg_stage_ctas_per_sm() : cg_stage_ctas_per_sm();
+    if (mix_) return cg_stage_mix_ctas_per_sm();
+    if (m.p.stage_split)
+        return tile_ == 8 ? ty8::cg_stage_split_ctas_per_sm() : cg_stage_split_ctas_per_sm();
+    return tile_ == 8 ? ty8::cg_stage_ctas_per_sm() : cg_stage_ctas_per_sm();
 }
 
 int Session::build_maps()
 {
-    auto tmap = [&](void *out, const float *base, int nf, bool halo) {
-        return tile_ == 8 ? ty8::make_field_tmap(out, base, g, nf, halo) : make_field_tmap(out, base, g, nf, halo);
+    auto tmap = [&](void *out, const float *base, int nf, bool halo, int box_nf = 0) {
+        return tile_ == 8 ? ty8::make_field_tmap(out, base, g, nf, halo, box_nf)
+                          : make_field_tmap(out, base, g, nf, halo, box_nf);
     };
     for (int b = 0; b < 3; b++) {
         CU(tmap(maps_[b].win, W_[b], 9, true));
         CU(tmap(maps_[b].winp, W_[b], 9, false));
-        CU(tmap(maps_[b].cjm, cjm_, 13, false));
+        CU(tmap(maps_[b].cjm, cjm_, 13, false, 3));
+        CU(tmap(maps_[b].cjm1, cjm_, 13, false, 1));
         CU(tmap(maps_[b].wm, W_[0], 9, false));
         CU(tmap(maps_[b].t, W_[3], 9, false));
     }
@@ -669,7 +675,8 @@ void Session::stage_desc_mix(int parity, int irk, CgStageDesc &d) const
     a.it_dev = it_dev_;
     a.zs_min = zs_min_, a.zp_max = zp_max_;
     make_field_tmap(d.tmW, A, g, 9, true);
-    make_field_tmap(d.tmC, cjm_, g, 13, false);
+    make_field_tmap(d.tmC, cjm_, g, 13, false, 3);
+    make_field_tmap(d.tmC1, cjm_, g, 13, false, 1);
     make_field_tmap(d.tmM, A, g, 9, false);
     make_field_tmap16(d.tmT, T16_, gh_, 9);
     make_field_tmap16(d.tmS, irk == 2 ? Sc_ : Sb_, gh_, 9);
