@@ -50,6 +50,12 @@ int Session::set_tiling(int kc, int ctas)
         err = "kchunk and ctas must be >= 1";
         return ST_ARG;
     }
+    tiling_chosen_ = true;
+    return apply_tiling(kc, ctas);
+}
+
+int Session::apply_tiling(int kc, int ctas)
+{
     kchunk_ = std::min(kc, m.g.nz);
     nchunk_ = (m.g.nz + kchunk_ - 1) / kchunk_;
     grid_ctas_ = (int)std::min<long long>(std::min(ctas, device_sms(device) * stage_ctas_per_sm()),

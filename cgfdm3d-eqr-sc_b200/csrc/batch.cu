@@ -87,6 +87,26 @@ int Batch::create(const std::vector<Session *> &sessions)
             err = x->err;
             return st;
         }
+    // one pencil length for the shared launch, from the tiles of all sessions
+    // (a small session's own is shorter); a session whose pencil was chosen
+    // by set_tiling or the autotuner keeps it
+    {
+        int nz = 1, sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        long long columns = 0;
+        for (Session *x : s) {
+            nz = std::max(nz, x->m.g.nz);
+            columns += (long long)x->stage_tiles() * x->m.g.nz;
+        }
+        const int per_sm = mix_ ? cg_stage_mix_ctas_per_sm() : cg_stage_ctas_per_sm();
+        const int k = stage_chunk((columns + nz - 1) / nz, nz, sms * per_sm);
+        for (Session *x : s)
+            if (!x->tiling_chosen())
+                if (int st = x->apply_tiling(k, 1 << 30)) {
+                    err = x->err;
+                    return st;
+                }
+    }
     BCU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     BCU(cudaEventCreate(&ev_[0]));
     BCU(cudaEventCreate(&ev_[1]));

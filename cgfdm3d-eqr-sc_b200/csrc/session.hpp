@@ -20,6 +20,9 @@ void fb_signs(int step, int fb[3]);
 void arena_session_add(int device);
 void arena_session_remove(int device);
 
+// planes per work item of a stage launch (csrc/session.cu)
+int stage_chunk(long long tiles, int nz, int ctas);
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -76,6 +79,8 @@ public:
     // planes per work item and persistent CTAs; autotune times candidates
     // on trial steps and keeps the fastest, the state restored after each
     int set_tiling(int kchunk, int ctas);
+    int apply_tiling(int kchunk, int ctas);         // the same without marking it as the caller's choice
+    bool tiling_chosen() const { return tiling_chosen_; }
     int autotune(int trial_steps, int *kchunk, int *ctas, float *ms_per_step);
     int kchunk() const { return kchunk_; }
     int ctas() const { return grid_ctas_; }
@@ -147,6 +152,7 @@ private:
     FaultDev fault_ = {};
     PointDev point_ = {};
     int kchunk_ = 8;
+    bool tiling_chosen_ = false;   // set_tiling was called: batches keep the pencil
     cudaGraphExec_t graph8_ = nullptr;
     cudaGraph_t graph8_src_ = nullptr;
     cudaEvent_t ev_[4] = {};
@@ -204,6 +210,7 @@ public:
     void stage_desc(int irk, CgStageDesc &d) const;
     void stage_desc_mix(int parity, int irk, CgStageDesc &d) const;
     int stage_items() const;
+    int stage_tiles() const { return ntx_ * nty_; }
     int pml_faces() const;
     int launch_sources_on(cudaStream_t st);
     int launch_stations_on(cudaStream_t st);
