@@ -174,7 +174,7 @@ int Session::adj_prepare()
     ALLOC(adj_.M, float, F * 9);
     ALLOC(adj_.Lam, float, F * 9);
     if (!m.p.adj_fused) {
-        ALLOC(adj_.Phi, float, F * 27);
+        ALLOC(adj_.Phi, float, F * 21);
         ALLOC(adj_.SF, float, g.plane * 36);
     } else {
         ALLOC(adj_.M2, float, F * 9);

@@ -225,7 +225,7 @@ struct AdjStageArgs {
     const float *Lp;     // lambda' (9 fields)
     float *M;            // mu_s in; mu_{s-1} out
     float *Lam;          // running sum; lambda_n after stage 0
-    float *Phi;          // 27 fields: per direction, the adjoint of its one-sided differences
+    float *Phi;          // 21 fields (phi_channel): per direction, the adjoint of its one-sided differences
     float *SF;           // surface layers L = 0..2 (k = _nz-1-L): 12 channels each, [3][12][plane]
     PmlFace face[5];     // adjoint auxiliaries per face: A = lambda', B = mu, T = running sum
     const float *h;      // stored RHS h_s of the forward stage (9 fields, HBox layout), or null: no gradient

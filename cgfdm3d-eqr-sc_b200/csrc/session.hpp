@@ -220,7 +220,7 @@ public:
 
 private:
     // adjoint state: lambda', mu, running sum (9 fields each), the per-
-    // direction difference adjoints (27 fields), the surface channels, the
+    // direction difference adjoints (21 fields), the surface channels, the
     // auxiliaries' adjoints per face, the gradient and d rdz / d (mu, lambda)
     struct Adjoint {
         float *Lp = nullptr, *M = nullptr, *Lam = nullptr, *Phi = nullptr, *SF = nullptr;
