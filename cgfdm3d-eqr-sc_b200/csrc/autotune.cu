@@ -59,7 +59,7 @@ int Session::apply_tiling(int kc, int ctas)
     kchunk_ = std::min(kc, m.g.nz);
     nchunk_ = (m.g.nz + kchunk_ - 1) / kchunk_;
     grid_ctas_ = (int)std::min<long long>(std::min(ctas, device_sms(device) * stage_ctas_per_sm()),
-                                          (long long)stage_items());
+                                          (long long)stage_units());
     if (int st = build_stage_descs()) return st;
     if (graph8_) cudaGraphExecDestroy(graph8_);
     if (graph8_src_) cudaGraphDestroy(graph8_src_);

@@ -132,7 +132,7 @@ int Batch::build_tables()
     for (int i = 0; i < n; i++) items[i + 1] = items[i] + s[i]->stage_items();
     std::vector<CgStageDesc> d(n);
     for (int irk = 0; irk < 4; irk++) {
-        for (int i = 0; i < n; i++) s[i]->stage_desc(irk, d[i]);
+        for (int i = 0; i < n; i++) s[i]->stage_desc(irk, d[i], true);
         BCU(cudaMemcpy(desc_[irk], d.data(), sizeof(CgStageDesc) * n, cudaMemcpyHostToDevice));
     }
     if (mix_)

@@ -29,14 +29,12 @@
 // Arithmetic follows the reference's expression order term by term; built
 // with --fmad=false the stage reproduces the reference's FP32 results bit for
 // bit, built normally it differs only by FMA contraction.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include <type_traits>
 
 #include "cg_ops.cuh"
 #include "device.cuh"
 #include "kernels.cuh"
+#include "tma.cuh"
 
 // L2 promotion of the plane-ring (halo) and point-operand tensor maps, and
 // which point operands are prefetched into L2 ahead of their loads.
@@ -189,8 +187,6 @@ static size_t stage2_smem()
     return (size_t)(NHSLOT * SLOT_SF + NCSLOT * CSLOT_SF + STASH_F) * 4 + (NHSLOT + NCSLOT) * 8;
 }
 
-// ------------------------------------------------------------ TMA helpers
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 // one float from global to shared memory, asynchronously (cp.async); this
 // thread waits for its own copies with cp_async_wait_all
 __device__ __forceinline__ void cp_async4(float *dst, const float *src)
@@ -199,55 +195,6 @@ __device__ __forceinline__ void cp_async4(float *dst, const float *src)
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity)
-{
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: gives up after `limit` clock cycles (2^31, about a second,
-// unless a test shortens it).
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned parity, long long limit)
-{
-    if (mbar_try_wait(bar, parity)) return true;
-    long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > limit) return false;
-    return true;
-}
-__device__ __forceinline__ void tma_load_4d(unsigned dst, const void *tmap, int x, int y, int z, int f, unsigned bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];\n" ::"r"(dst),
-        "l"((unsigned long long)tmap), "r"(x), "r"(y), "r"(z), "r"(f), "r"(bar)
-        : "memory");
-}
-
-__device__ __forceinline__ void l2_prefetch(const void *p)
-{
-    asm volatile("prefetch.global.L2 [%0];\n" ::"l"((unsigned long long)p));
-}
-__device__ __forceinline__ void tma_prefetch_4d(const void *tmap, int x, int y, int z, int f)
-{
-    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(
-                     (unsigned long long)tmap),
-                 "r"(x), "r"(y), "r"(z), "r"(f)
-                 : "memory");
-}
 
 // Stencil taps: hc points at this thread's cell of the current plane's halo
 // box (x and y derivatives), zp[m] at its cell of plane k + FB3*(m-1) for the
@@ -466,7 +413,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
     constexpr int hyL = FB2 > 0 ? 1 : 3;
     constexpr int za = FB3 > 0 ? 1 : 3;
     const int cell = (ty + hyL) * BXW + tx + 4;
-    const int total = BATCH ? item_start[nsess] : d1.a.ntiles_x * d1.a.ntiles_y * d1.a.nchunk;
+    const int total = BATCH ? item_start[nsess] : d1.a.ntiles_x * d1.a.ntiles_y * d1.a.nchunk * (V2 ? d1.a.sweeps : 1);
     int sess = -1;
     // mixed storage (one thread): per-field scales of this step from the
     // bounds of the session's step-start state -- the bound of field f
@@ -519,6 +466,9 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
 #pragma unroll
     for (int f = 0; f < (MIX ? 9 : 1); f++) rm[f] = 0.0f;
 
+    // The split pipeline's items may be `sweeps` tiles high; their sweeps are
+    // handed out one by one, so the sweeps of an item run side by side.
+    const int sweeps = V2 ? d1.a.sweeps : 1;
     for (;;) {
     __syncthreads();
     if (tid == 0) s_item = atomicAdd(&work[0], 1);
@@ -580,15 +530,16 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                    (long long)kp * g.nx * nPML;
         return (long long)ip + (long long)jp * g.nx + (long long)kp * g.nx * g.ny;
     };
-    const int item = BATCH ? gitem - item_start[sess] : gitem;
+    const int item = BATCH ? gitem - item_start[sess] : V2 ? gitem / sweeps : gitem;
+    const int sweep = V2 ? gitem - item * sweeps : 0;
     const int tile = item / a.nchunk, chunk = item - tile * a.nchunk;
     const int by_ = tile / a.ntiles_x, bx_ = tile - by_ * a.ntiles_x;
-    const int i0 = CGFDM_HALO + bx_ * TX, j0 = CGFDM_HALO + by_ * TY;
+    const int i0 = CGFDM_HALO + bx_ * TX, j0 = CGFDM_HALO + (by_ * sweeps + sweep) * TY;
     const int i = i0 + tx, j = j0 + ty;
     const bool active = i < _nx && j < _ny;
     const int kb = CGFDM_HALO + chunk * a.kchunk;
     const int ke = min(kb + a.kchunk, _nz);
-    if (kb >= ke) continue;
+    if (kb >= ke || j0 >= _ny) continue;
     const int kf = kb - za;                 // first plane this item loads
     const int tx0 = g.xoff + i0 - 4;        // halo box origin column: a multiple of 4 (16 bytes)
     const int ty0 = j0 - hyL;
@@ -613,7 +564,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
         unsigned bar = smem_u32(cbar(s));
         // test hook: leave this plane's slot without a copy (and without the
         // arrival that would complete its barrier phase), once
-        if (a.stall && gitem == a.stall_item && kk - kf == a.stall_fill && atomicExch(a.stall, 0) == 1) return;
+        if (a.stall && (BATCH ? gitem : item) == a.stall_item && sweep == 0 && kk - kf == a.stall_fill && atomicExch(a.stall, 0) == 1) return;
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         if constexpr (MIX) {
             const bool hs = irk != 0;
@@ -1210,14 +1161,8 @@ size_t cg_stage2_smem_bytes() { return stage2_smem(); }
 #if CG_TILE_Y == 4
 cudaError_t make_field_tmap16(void *out, const __half *base, const DevGrid &gh, int nf)
 {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (!encode) {
-        cudaDriverEntryPointQueryResult q;
-        void *fn = nullptr;
-        CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-        if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
-        encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-    }
+    const auto encode = tmap_encoder();
+    if (!encode) return cudaErrorNotSupported;
     cuuint64_t dims[4] = {(cuuint64_t)gh.pitch, (cuuint64_t)gh.nyp, (cuuint64_t)gh.nzp, (cuuint64_t)nf};
     cuuint64_t strides[3] = {(cuuint64_t)gh.pitch * 2, (cuuint64_t)gh.plane * 2, (cuuint64_t)gh.fstride * 2};
     cuuint32_t box[4] = {(cuuint32_t)BXW, (cuuint32_t)BYW, 1, (cuuint32_t)nf};
@@ -1279,14 +1224,8 @@ cudaError_t launch_cg_stage_batch(int FB1, int FB2, int FB3, int irk, const CgSt
 
 cudaError_t make_field_tmap(void *out, const float *base, const DevGrid &g, int nf, bool halo_box, int box_nf)
 {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (!encode) {
-        cudaDriverEntryPointQueryResult q;
-        void *fn = nullptr;
-        CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-        if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
-        encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-    }
+    const auto encode = tmap_encoder();
+    if (!encode) return cudaErrorNotSupported;
     cuuint64_t dims[4] = {(cuuint64_t)g.pitch, (cuuint64_t)g.nyp, (cuuint64_t)g.nzp, (cuuint64_t)nf};
     cuuint64_t strides[3] = {(cuuint64_t)g.pitch * 4, (cuuint64_t)g.plane * 4, (cuuint64_t)g.fstride * 4};
     cuuint32_t box[4] = {halo_box ? (cuuint32_t)BXW : (cuuint32_t)TX, halo_box ? (cuuint32_t)BYW : (cuuint32_t)TY, 1,

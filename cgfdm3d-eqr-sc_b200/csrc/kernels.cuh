@@ -98,6 +98,7 @@ struct CgStageArgs {
     const int *it_dev;
     float zs_min, zp_max;
     int ntiles_x, ntiles_y, nchunk;  // work items: tiles x tiles x z-chunks
+    int sweeps;          // split pipeline: 4-row column sweeps an item is high (its tile rows / 4)
     int irk;
     int FB1, FB2, FB3;
     int nPML;
@@ -135,7 +136,8 @@ struct alignas(64) CgStageDesc {
 // item_start[s] .. item_start[s+1]-1, its descriptor is descs[s] in device
 // memory; all advance with the same FB signs and stage number.
 // launch_cg_stage_split: the split pipeline (the current plane's halo box,
-// interior column boxes for the z window): one session's FP32 stage.
+// interior column boxes for the z window): one session's FP32 stage, a.sweeps
+// 4-row sweeps an item (namespace ty4 only).
 // launch_cg_stage_mix: mixed-precision storage (the MIX instantiation);
 // launch_cg_stage_batch_mix: the same for a batch of such sessions.
 // make_field_tmap16: FP16 counterpart of make_field_tmap (halo box), for

@@ -493,7 +493,7 @@ int Session::setup_device()
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device);
     ntx_ = (G.nx + 31) / 32;
     nty_ = (G.ny + tile_ - 1) / tile_;
-    const long long tiles = (long long)ntx_ * nty_;
+    const long long tiles = (long long)ntx_ * nty_ * (split() ? tile_ / 4 : 1);
     const int ctas = dev_sms * stage_ctas_per_sm();
     kchunk_ = stage_chunk(tiles, G.nz, ctas);
     nchunk_ = (G.nz + kchunk_ - 1) / kchunk_;
@@ -545,7 +545,7 @@ int stage_chunk(long long tiles, int nz, int ctas)
 
 // The four stage descriptors (RK4 stage irk reads win[irk] and writes
 // wout[irk]: A -> B, B -> C, C -> B, B -> A) with their tensor maps.
-void Session::stage_desc(int irk, CgStageDesc &d) const
+void Session::stage_desc(int irk, CgStageDesc &d, bool batched) const
 {
     float *A = W_[0], *B = W_[1], *C = W_[2], *T = W_[3];
     const float *win[4] = {A, B, C, B};
@@ -579,16 +579,20 @@ void Session::stage_desc(int irk, CgStageDesc &d) const
     a.stall_fill = stall_fill_;
     a.wait_limit = wait_limit_;
     a.ntiles_x = ntx_, a.ntiles_y = nty_, a.nchunk = nchunk_;
+    a.sweeps = tile_ / 4;
     for (int f = 0; f < 6; f++) a.ho[f] = ho_[irk][f];
-    std::memcpy(d.tmW, maps_[win_map[irk]].win, 128);
-    std::memcpy(d.tmC, maps_[win_map[irk]].cjm, 128);
-    std::memcpy(d.tmC1, maps_[win_map[irk]].cjm1, 128);
-    std::memcpy(d.tmM, maps_[win_map[irk]].wm, 128);
-    std::memcpy(d.tmT, maps_[win_map[irk]].t, 128);
-    std::memcpy(d.tmWc, maps_[win_map[irk]].winp, 128);
+    const CgStageMaps &M = (split() && !batched ? split_maps_ : maps_)[win_map[irk]];
+    std::memcpy(d.tmW, M.win, 128);
+    std::memcpy(d.tmC, M.cjm, 128);
+    std::memcpy(d.tmC1, M.cjm1, 128);
+    std::memcpy(d.tmM, M.wm, 128);
+    std::memcpy(d.tmT, M.t, 128);
+    std::memcpy(d.tmWc, M.winp, 128);
 }
 
+// (the split pipeline hands an item's 4-row sweeps out one by one)
 int Session::stage_items() const { return ntx_ * nty_ * nchunk_; }
+int Session::stage_units() const { return stage_items() * (split() ? tile_ / 4 : 1); }
 
 // Absorbing faces as stage-kernel bits x1 y1 z1 x2 y2 (PML off: none).
 int Session::pml_faces() const
@@ -601,24 +605,29 @@ int Session::pml_faces() const
 int Session::stage_ctas_per_sm() const
 {
     if (mix_) return cg_stage_mix_ctas_per_sm();
-    if (m.p.stage_split)
-        return tile_ == 8 ? ty8::cg_stage_split_ctas_per_sm() : cg_stage_split_ctas_per_sm();
+    if (split()) return cg_stage_split_ctas_per_sm();
     return tile_ == 8 ? ty8::cg_stage_ctas_per_sm() : cg_stage_ctas_per_sm();
 }
 
+// Tensor maps of the stencil inputs: for the ring kernel (batches) boxes of
+// the tile height, for the split pipeline's own launches of its 4-row sweeps.
 int Session::build_maps()
 {
-    auto tmap = [&](void *out, const float *base, int nf, bool halo, int box_nf = 0) {
-        return tile_ == 8 ? ty8::make_field_tmap(out, base, g, nf, halo, box_nf)
-                          : make_field_tmap(out, base, g, nf, halo, box_nf);
-    };
-    for (int b = 0; b < 3; b++) {
-        CU(tmap(maps_[b].win, W_[b], 9, true));
-        CU(tmap(maps_[b].winp, W_[b], 9, false));
-        CU(tmap(maps_[b].cjm, cjm_, 13, false, 3));
-        CU(tmap(maps_[b].cjm1, cjm_, 13, false, 1));
-        CU(tmap(maps_[b].wm, W_[0], 9, false));
-        CU(tmap(maps_[b].t, W_[3], 9, false));
+    for (int split_set = 0; split_set < 2; split_set++) {
+        const bool eight = !split_set && tile_ == 8;
+        auto tmap = [&](void *out, const float *base, int nf, bool halo, int box_nf = 0) {
+            return eight ? ty8::make_field_tmap(out, base, g, nf, halo, box_nf)
+                         : make_field_tmap(out, base, g, nf, halo, box_nf);
+        };
+        for (int b = 0; b < 3; b++) {
+            CgStageMaps &M = (split_set ? split_maps_ : maps_)[b];
+            CU(tmap(M.win, W_[b], 9, true));
+            CU(tmap(M.winp, W_[b], 9, false));
+            CU(tmap(M.cjm, cjm_, 13, false, 3));
+            CU(tmap(M.cjm1, cjm_, 13, false, 1));
+            CU(tmap(M.wm, W_[0], 9, false));
+            CU(tmap(M.t, W_[3], 9, false));
+        }
     }
     return ST_OK;
 }
@@ -638,7 +647,7 @@ int Session::set_tile(int rows)
     nty_ = (m.g.ny + tile_ - 1) / tile_;
     int dev_sms = 148;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device);
-    grid_ctas_ = (int)std::min<long long>((long long)dev_sms * stage_ctas_per_sm(), (long long)stage_items());
+    grid_ctas_ = (int)std::min<long long>((long long)dev_sms * stage_ctas_per_sm(), (long long)stage_units());
     if (int st = build_maps()) return st;
     if (int st = build_stage_descs()) return st;
     if (graph8_) cudaGraphExecDestroy(graph8_);
@@ -651,9 +660,8 @@ int Session::set_tile(int rows)
 int Session::launch_stage(int FB1, int FB2, int FB3, const CgStageDesc &d)
 {
     cudaError_t e;
-    if (m.p.stage_split && !mix_)
-        e = tile_ == 8 ? ty8::launch_cg_stage_split(FB1, FB2, FB3, d, work_dev_, grid_ctas_, stream)
-                       : launch_cg_stage_split(FB1, FB2, FB3, d, work_dev_, grid_ctas_, stream);
+    if (split())
+        e = launch_cg_stage_split(FB1, FB2, FB3, d, work_dev_, grid_ctas_, stream);
     else
         e = tile_ == 8 ? ty8::launch_cg_stage(FB1, FB2, FB3, d, work_dev_, grid_ctas_, stream)
                        : launch_cg_stage(FB1, FB2, FB3, d, work_dev_, grid_ctas_, stream);
@@ -907,6 +915,9 @@ int Session::test_stall(int item, int fill, long long wait_cycles)
         err = "the stall hook applies to the CGFDM stage kernel";
         return ST_OPTIONS;
     }
+    // an item must hold that copy: its planes and the four of its first window
+    if (fill - 3 > kchunk_ && fill - 3 <= m.g.nz)
+        if (int st = apply_tiling(fill - 3, grid_ctas_)) return st;
     if (item < 0 || item >= stage_items() || fill < 0 || wait_cycles < 0) {
         err = "stall hook: item, fill or wait_cycles out of range";
         return ST_ARG;

@@ -156,7 +156,7 @@ private:
     cudaGraphExec_t graph8_ = nullptr;
     cudaGraph_t graph8_src_ = nullptr;
     cudaEvent_t ev_[4] = {};
-    CgStageMaps maps_[3] = {};                       // TMA descriptors per stencil input A, B, C
+    CgStageMaps maps_[3] = {}, split_maps_[3] = {};  // TMA descriptors per stencil input A, B, C
     CgStageDesc desc_host_[4] = {};                  // stage descriptors, one per RK stage
     int build_stage_descs();
     int *work_dev_ = nullptr;                        // persistent-CTA work counters
@@ -181,6 +181,7 @@ private:
     int tile_ = 4;
     int build_maps();                                // tensor maps of the stencil inputs for tile_
     int stage_ctas_per_sm() const;
+    bool split() const { return m.p.stage_split && !mix_ && !part_session_; }   // the split pipeline's kernel
     int *stall_dev_ = nullptr;                       // test hook of the stage kernel's bounded waits
     int stall_item_ = -1, stall_fill_ = 0;
     long long wait_limit_ = 0;
@@ -207,9 +208,10 @@ public:
     // the stage descriptor of RK stage irk (with FP16 storage: for the
     // step-start state of step parity `parity`), and the stage's work items
     // (batches use these)
-    void stage_desc(int irk, CgStageDesc &d) const;
+    void stage_desc(int irk, CgStageDesc &d, bool batched = false) const;
     void stage_desc_mix(int parity, int irk, CgStageDesc &d) const;
     int stage_items() const;
+    int stage_units() const;      // what the launch's counter hands out
     int stage_tiles() const { return ntx_ * nty_; }
     int pml_faces() const;
     int launch_sources_on(cudaStream_t st);
