@@ -42,6 +42,7 @@
 // the flux-difference corrections into one six-tap filter.
 #include "device.cuh"
 #include "kernels.cuh"
+#include "pair.cuh"
 #include "sc_ops.cuh"
 
 // 1: the passes' RHS and stage-output stores evict-first (each is read back
@@ -67,79 +68,104 @@ namespace {
 
 constexpr int SC_THREADS = 256;
 
-// ------------------------------------------------------------ WENO5-JS
+// ------------------------------------------------- two points at a time
 #ifndef CGFDM_EXACT
-__device__ __forceinline__ float rcp_approx(float x)
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return vadd(a, b); }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return vsub(a, b); }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return vmul(a, b); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return vfma(a, b, c); }
+__device__ __forceinline__ F2 rcp2(F2 x)
 {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
+    float a, b;
+    unpk(x, a, b);
+    asm("rcp.approx.f32 %0, %0;" : "+f"(a));
+    asm("rcp.approx.f32 %0, %0;" : "+f"(b));
+    return pk(a, b);
 }
-#endif
 
-// Both states upwinded from the cell centred at c, window a b c d e:
-// uL at the face c+1/2, uR at the face c-1/2.
+// -1 / x
+__device__ __forceinline__ F2 rcp2_neg(F2 x)
+{
+    float a, b;
+    unpk(x, a, b);
+    return rcp2(pk(-a, -b));
+}
+
+// ------------------------------------------------------------ WENO5-JS
+// Both states upwinded from the cell centred at c, window a b c d e: uL at
+// the face c+1/2, uR at the face c-1/2.  They share the Jiang-Shu indicators
+// of the sub-stencils (a,b,c), (b,c,d), (c,d,e), 13/12 s^2 + 1/4 t^2 + 1e-6
+// with s the second difference and t the slope, here times 12/13 (a common
+// factor of the indicators cancels in the weights).  Everything is written in
+// the cell differences d0..d3: the sub-stencils' states are c + q / 8 (uL)
+// and c - q / 8 (uR), their weights 5/16, 10/16, 1/16 taken times 16/5.
+__device__ __forceinline__ void weno_pair(F2 a, F2 b, F2 c, F2 d, F2 e, F2 &uL, F2 &uR)
+{
+    const F2 two = pk(2.0f), three = pk(3.0f), four = pk(4.0f), eight = pk(8.0f), fifth = pk(0.2f);
+    const F2 k = pk(3.0f / 13.0f), eps = pk(1e-6f * 12.0f / 13.0f);
+    const F2 d0 = b - a, d1 = c - b, d2 = d - c, d3 = e - d;
+    const F2 s0 = d1 - d0, s1 = d2 - d1, n2 = d2 - d3;   // n2: minus the third second difference
+    const F2 t0 = fma2(two, d1, s0), t1 = fma2(two, d1, s1), t2 = fma2(two, d2, n2);
+    const F2 B0 = fma2(s0, s0, fma2(k * t0, t0, eps));
+    const F2 B1 = fma2(s1, s1, fma2(k * t1, t1, eps));
+    const F2 B2 = fma2(n2, n2, fma2(k * t2, t2, eps));
+    const F2 r0 = rcp2(B0 * B0), r1 = rcp2(B1 * B1), r2 = rcp2(B2 * B2);
+    const F2 wm = two * r1, far0 = fifth * r0, far2 = fifth * r2;
+    // q of the face-side, centred and far sub-stencils
+    const F2 nL = fma2(r2, fma2(four, d2, n2), fma2(wm, fma2(three, d2, d1), far0 * fma2(two, t0, s0)));
+    const F2 nR = fma2(r0, fma2(four, d1, s0), fma2(wm, fma2(three, d1, d2), far2 * fma2(two, t2, n2)));
+    const F2 m = eight * wm;
+    uL = fma2(nL, rcp2(fma2(eight, r2, fma2(eight, far0, m))), c);
+    uR = fma2(nR, rcp2_neg(fma2(eight, r0, fma2(eight, far2, m))), c);
+}
+
+// Lax-Friedrichs flux of a face from its left (uL) and right (uR) states,
+// n the metric row's terms that are not zero on a grid of vertical columns
+// (n[0]: y_eta z_zeta for xi, x_xi z_zeta for eta; all three for zeta).  The
+// flux is linear in the state: f(uL) + f(uR) = f(uL + uR).
+template <int DIR>
+__device__ __forceinline__ void lf_flux(const F2 n[3], F2 lam, F2 mu, F2 buo, F2 ha, const F2 uL[9], const F2 uR[9],
+                                        F2 F[9])
+{
+    F2 s[9];
+    const F2 half = pk(-0.5f);
+#pragma unroll
+    for (int v = 0; v < 9; v++) {
+        s[v] = uL[v] + uR[v];
+        F[v] = ha * (uL[v] - uR[v]);
+    }
+    const F2 ltr = lam * ((s[3] + s[4]) + s[5]), m2 = mu + mu;
+    const F2 n0 = half * n[0];
+    if constexpr (DIR == 0) {
+        const F2 nm = n0 * mu, nb = n0 * buo;
+        F[0] = fma2(n0, fma2(m2, s[3], ltr), F[0]);
+        F[1] = fma2(nm, s[8], F[1]), F[2] = fma2(nm, s[7], F[2]);
+        F[3] = fma2(nb, s[0], F[3]), F[7] = fma2(nb, s[2], F[7]), F[8] = fma2(nb, s[1], F[8]);
+    } else if constexpr (DIR == 1) {
+        const F2 nm = n0 * mu, nb = n0 * buo;
+        F[1] = fma2(n0, fma2(m2, s[4], ltr), F[1]);
+        F[0] = fma2(nm, s[8], F[0]), F[2] = fma2(nm, s[6], F[2]);
+        F[4] = fma2(nb, s[1], F[4]), F[6] = fma2(nb, s[2], F[6]), F[8] = fma2(nb, s[0], F[8]);
+    } else {
+        const F2 n1 = half * n[1], n2 = half * n[2];
+        const F2 m0 = n0 * mu, m1 = n1 * mu, mm2 = n2 * mu, b0 = n0 * buo, b1 = n1 * buo, b2 = n2 * buo;
+        F[0] = fma2(n0, fma2(m2, s[3], ltr), fma2(m1, s[8], fma2(mm2, s[7], F[0])));
+        F[1] = fma2(n1, fma2(m2, s[4], ltr), fma2(m0, s[8], fma2(mm2, s[6], F[1])));
+        F[2] = fma2(n2, fma2(m2, s[5], ltr), fma2(m0, s[7], fma2(m1, s[6], F[2])));
+        F[3] = fma2(b0, s[0], F[3]), F[4] = fma2(b1, s[1], F[4]), F[5] = fma2(b2, s[2], F[5]);
+        F[6] = fma2(b1, s[2], fma2(b2, s[1], F[6]));
+        F[7] = fma2(b0, s[2], fma2(b2, s[0], F[7]));
+        F[8] = fma2(b0, s[1], fma2(b1, s[0], F[8]));
+    }
+}
+#else
+// The reference's states and flux, term by term.
 __device__ __forceinline__ void weno_pair(float a, float b, float c, float d, float e, float &uL, float &uR)
 {
-#ifdef CGFDM_EXACT
     uL = weno5_ref(a, b, c, d, e);
     uR = weno5_ref(e, d, c, b, a);
-#else
-    // Jiang-Shu indicators over the cell of c for the sub-stencils
-    // (a,b,c), (b,c,d), (c,d,e): 13/12 (second difference)^2 + 1/4 (slope)^2
-    const float k13 = 13.0f / 12.0f;
-    const float s0 = (a - 2.0f * b) + c, t0 = (a - 4.0f * b) + 3.0f * c;
-    const float s1 = (b - 2.0f * c) + d, t1 = b - d;
-    const float s2 = (c - 2.0f * d) + e, t2 = (3.0f * c - 4.0f * d) + e;
-    const float B0 = k13 * s0 * s0 + 0.25f * t0 * t0 + 1e-6f;
-    const float B1 = k13 * s1 * s1 + 0.25f * t1 * t1 + 1e-6f;
-    const float B2 = k13 * s2 * s2 + 0.25f * t2 * t2 + 1e-6f;
-    const float r0 = rcp_approx(B0 * B0), r1 = rcp_approx(B1 * B1), r2 = rcp_approx(B2 * B2);
-    // linear weights 5/16, 10/16, 1/16 for the sub-stencil on the face side,
-    // the centred one and the far one (the common 1/16 cancels)
-    {
-        const float wa = 5.0f * r2, wb = 10.0f * r1, wc = r0;
-        const float qa = 0.375f * c + 0.75f * d - 0.125f * e;
-        const float qb = -0.125f * b + 0.75f * c + 0.375f * d;
-        const float qc = 0.375f * a - 1.25f * b + 1.875f * c;
-        uL = (wa * qa + wb * qb + wc * qc) * rcp_approx(wa + wb + wc);
-    }
-    {
-        const float wa = 5.0f * r0, wb = 10.0f * r1, wc = r2;
-        const float qa = 0.375f * c + 0.75f * b - 0.125f * a;
-        const float qb = -0.125f * d + 0.75f * c + 0.375f * b;
-        const float qc = 0.375f * e - 1.25f * d + 1.875f * c;
-        uR = (wa * qa + wb * qb + wc * qc) * rcp_approx(wa + wb + wc);
-    }
-#endif
 }
-
-// Lax-Friedrichs flux of a face from its left (uL) and right (uR) states.
-__device__ __forceinline__ void lf_flux(float n0, float n1, float n2, float lam, float mu, float buo, float alpha,
-                                        const float uL[9], const float uR[9], float F[9])
-{
-#ifdef CGFDM_EXACT
-    lf_flux_ref(n0, n1, n2, lam, mu, buo, alpha, uL, uR, F);
-#else
-    // the flux is linear in the state: f(uL) + f(uR) = f(uL + uR)
-    float s[9], fs[9];
-#pragma unroll
-    for (int v = 0; v < 9; v++) s[v] = uL[v] + uR[v];
-    const float tr = s[3] + s[4] + s[5], m2 = 2.0f * mu;
-    fs[0] = n0 * (lam * tr + m2 * s[3]) + mu * (n1 * s[8] + n2 * s[7]);
-    fs[1] = n1 * (lam * tr + m2 * s[4]) + mu * (n0 * s[8] + n2 * s[6]);
-    fs[2] = n2 * (lam * tr + m2 * s[5]) + mu * (n0 * s[7] + n1 * s[6]);
-    fs[3] = buo * (n0 * s[0]);
-    fs[4] = buo * (n1 * s[1]);
-    fs[5] = buo * (n2 * s[2]);
-    fs[6] = buo * (n1 * s[2] + n2 * s[1]);
-    fs[7] = buo * (n0 * s[2] + n2 * s[0]);
-    fs[8] = buo * (n0 * s[1] + n1 * s[0]);
-    const float ha = 0.5f * alpha;
-#pragma unroll
-    for (int v = 0; v < 9; v++) F[v] = -0.5f * fs[v] - ha * (uR[v] - uL[v]);
 #endif
-}
 
 // Exponential-decay factor product of an interior point, in the
 // reference's order x-low, x-high, y-low, y-high, z-low
@@ -206,21 +232,6 @@ __device__ __noinline__ void surface_diff(const ScDirArgs &a, long long q, long 
     }
 }
 
-// Flux difference of an interior point from the fluxes f[0..5] of the faces
-// p-5/2 .. p+5/2 (src/alternative_flux_FD.cpp:1283).
-__device__ __forceinline__ float interior_diff(const float f[6], float coef)
-{
-#ifdef CGFDM_EXACT
-    return interior_diff_ref(f, coef);
-#else
-    // corrected face flux Fh = c2 F-2 + c1 F-1 + c0 F0 + c1 F+1 + c2 F+2 with
-    // c0 = 6402/5760, c1 = -348/5760, c2 = 27/5760; val = -coef (Fh[p] - Fh[p-1])
-    // = coef (c2 (F[p-3] - F[p+2]) + (c1 - c2) (F[p-2] - F[p+1]) + (c0 - c1) (F[p-1] - F[p]))
-    constexpr float e0 = 27.0f / 5760, e1 = (-348.0f - 27.0f) / 5760, e2 = (6402.0f + 348.0f) / 5760;
-    return coef * (e0 * (f[0] - f[5]) + e1 * (f[1] - f[4]) + e2 * (f[2] - f[3]));
-#endif
-}
-
 // The pass's use of the flux difference val of point q = (i, j, k): the x
 // pass stores the RHS, the y pass adds to it, the z pass adds its part and
 // applies the TVD-RK3 update (src/wave_rk_tvd.cpp:17-78), the sponge below
@@ -265,6 +276,70 @@ __device__ __forceinline__ void epilogue(const ScDirArgs &a, long long q, int i,
     }
 }
 
+#ifndef CGFDM_EXACT
+// The same for two neighbouring points (rows j, j+1 of the x pass, columns
+// i, i+1 of the others); two: the second one is inside the grid.
+template <int DIR>
+__device__ __forceinline__ void epilogue2(const ScDirArgs &a, long long q, int i, int j, int k, bool two,
+                                          const F2 val[9])
+{
+    const long long F = a.g.fstride;
+    auto ld = [&](const float *p) { return SC_LD(*reinterpret_cast<const float2 *>(p)); };
+    auto st = [&](float *p, float x, float y) {
+        if (two) SC_ST(*reinterpret_cast<float2 *>(p), make_float2(x, y));
+        else SC_ST(*p, x);
+    };
+    if (DIR == 0) {
+#pragma unroll
+        for (int v = 0; v < 9; v++) {
+            float x, y;
+            unpk(val[v], x, y);
+            SC_ST(a.H[v * F + q], x);
+            if (two) SC_ST(a.H[v * F + q + a.g.pitch], y);
+        }
+    } else if (DIR == 1) {
+        F2 h[9];
+#pragma unroll
+        for (int v = 0; v < 9; v++) {
+            const float2 w = ld(a.H + v * F + q);
+            h[v] = pk(w.x, w.y) + val[v];
+        }
+#pragma unroll
+        for (int v = 0; v < 9; v++) {
+            float x, y;
+            unpk(h[v], x, y);
+            st(a.H + v * F + q, x, y);
+        }
+    } else {
+        const int _nz = a.g.nzp - CGFDM_HALO;
+        const bool decay = a.decay != nullptr && k < _nz - 4;
+        auto rk = [&](float m, float w, float h) -> float {
+            if (a.irk == 1)
+                return __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(0.75, (double)m), __dmul_rn(0.25, (double)w)),
+                                                   __dmul_rn(0.25, (double)h)));
+            return __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(1.0 / 3.0, (double)m),
+                                                         __dmul_rn(2.0 / 3.0, (double)w)),
+                                               __dmul_rn(2.0 / 3.0, (double)h)));
+        };
+#pragma unroll 3
+        for (int v = 0; v < 9; v++) {
+            const float2 h0 = ld(a.H + v * F + q), w = *reinterpret_cast<const float2 *>(a.W + v * F + q);
+            float2 m = make_float2(0.0f, 0.0f), o;
+            if (a.irk != 0) m = ld(a.Wm + v * F + q);
+            float hx, hy;
+            unpk(pk(h0.x, h0.y) + val[v], hx, hy);
+            if (a.irk == 0) o.x = w.x + hx, o.y = w.y + hy;
+            else o.x = rk(m.x, w.x, hx), o.y = rk(m.y, w.y, hy);
+            if (decay) {
+                o.x = decay_apply(o.x, i, j, k, a.g, a.decay, a.ndecay);
+                o.y = decay_apply(o.y, i + 1, j, k, a.g, a.decay, a.ndecay);
+            }
+            st(a.Wout + v * F + q, o.x, o.y);
+        }
+    }
+}
+#endif
+
 // ------------------------------------------------------------ tiled pass
 // Tiles of NPOS positions along the pass direction (the tile's NPOS - 6
 // points and the neighbours their differences reach) times NL lanes across
@@ -274,28 +349,125 @@ __device__ __forceinline__ void epilogue(const ScDirArgs &a, long long q, int i,
 //   A  both WENO states upwinded from every position,
 //   B  the Lax-Friedrichs flux of every face, written over the left states,
 //   C  the flux difference of every point and the pass's epilogue.
+//
+// The default build gives each of the 256 threads one position of two
+// neighbouring lanes, packed (F2): 64 positions x 8 rows, 32 positions x 16
+// columns.  The build that rounds every operation takes a lane at a time, in
+// the reference's order.
+#ifndef CGFDM_EXACT
+constexpr int SCX_NPOS = 64, SCX_NL = 8;
+#else
 constexpr int SCX_NPOS = 64, SCX_NL = 4;
-// y and z tiles: 32 positions (26 points) x 16 columns, 37 KB of shared
-// memory, five CTAs per SM (register cap 48); on the 512 x 512 x 256 basin
-// workload this beat 80 x 16 at two CTAs by 1.4x and a one-warp-per-pencil
-// register-streaming variant by 1.7x: the passes are latency-bound and
-// occupancy pays (staging the W window in shared memory first, at three to
-// five CTAs per SM, was 1.5x slower than reading it through L1, and sliding
-// one thread's window over two positions 6 % slower than one position per
-// thread).
-#ifndef SCY_NPOS
-#define SCY_NPOS 32
 #endif
-#ifndef SCY_NL
-#define SCY_NL 16
-#endif
-
+constexpr int SCY_NPOS = 32, SCY_NL = 16;
 #ifndef SC_TILE_MIN_CTAS
-#define SC_TILE_MIN_CTAS 5
+#define SC_TILE_MIN_CTAS 3
 #endif
 // shared memory of a tile: left and right states, 9 + 9 fields per position
 constexpr size_t sc_tile_smem(int npos, int nl) { return sizeof(float) * 18 * npos * nl; }
 
+#ifndef CGFDM_EXACT
+template <int DIR, int NPOS, int NL>
+__global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const ScDirArgs a)
+{
+    constexpr int PR = NL / 2;                     // lane pairs
+    constexpr int STEP = DIR == 0 ? 1 : PR;        // threads from one position to the next
+    static_assert(NPOS * PR == SC_THREADS, "one position of one lane pair a thread");
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    F2 *sL = reinterpret_cast<F2 *>(sm_raw), *sR = sL + 9 * SC_THREADS;
+    const DevGrid &g = a.g;
+    const long long F = g.fstride;
+    const int _nx = g.nxp - CGFDM_HALO, _ny = g.nyp - CGFDM_HALO, _nz = g.nzp - CGFDM_HALO;
+    const int nd = DIR == 0 ? _nx : DIR == 1 ? _ny : _nz;  // points along the pass end before nd
+    const long long stride = DIR == 0 ? 1 : DIR == 1 ? (long long)g.pitch : g.plane;
+    const int tile = DIR == 0 ? blockIdx.x : DIR == 1 ? blockIdx.y : blockIdx.z;
+    const int lane_end = DIR == 0 ? _ny : _nx;
+    const int t = threadIdx.x;
+    const int mi = DIR == 0 ? t % NPOS : t / PR, pr = DIR == 0 ? t / NPOS : t % PR;
+    const int m = tile * (NPOS - 6) + mi;                                           // padded index along the pass
+    const int lane = CGFDM_HALO + (DIR == 0 ? blockIdx.y : blockIdx.x) * NL + 2 * pr;
+    const int i = DIR == 0 ? m : lane, j = DIR == 0 ? lane : DIR == 1 ? m : CGFDM_HALO + (int)blockIdx.y,
+              k = DIR == 2 ? m : CGFDM_HALO + (int)blockIdx.z;
+    // the pair's second lane may be the first halo lane of a row (read, never
+    // written); columns lie on 8-byte boundaries (xoff 1, tiles of 16)
+    const bool have = lane < lane_end, two = lane + 1 < lane_end;
+    const long long q = g.at(i, j, k);
+    auto ld = [&](const float *p) -> F2 {
+        if constexpr (DIR == 0) return pk(__ldg(p), __ldg(p + g.pitch));
+        else {
+            const float2 w = __ldg(reinterpret_cast<const float2 *>(p));
+            return pk(w.x, w.y);
+        }
+    };
+    // ---- phase A: both WENO states of every position
+    const bool face = have && mi < NPOS - 1 && m >= 2 && m < nd;
+    F2 n[3], lam, mu, buo;
+    if (face) {
+        if constexpr (DIR < 2) n[0] = ld(a.cjm + (DIR == 0 ? C_XI_X : C_ET_Y) * F + q);
+        else n[0] = ld(a.cjm + C_ZT_X * F + q), n[1] = ld(a.cjm + C_ZT_Y * F + q), n[2] = ld(a.cjm + C_ZT_Z * F + q);
+        lam = ld(a.cjm + C_LAMBDA * F + q), mu = ld(a.cjm + C_MU * F + q), buo = ld(a.cjm + C_BUOY * F + q);
+    }
+    if (have && m >= 2 && m <= nd) {
+        const float *w = a.W + q;
+#pragma unroll 3
+        for (int v = 0; v < 9; v++) {
+            const float *wv = w + v * F;
+            weno_pair(ld(wv - 2 * stride), ld(wv - stride), ld(wv), ld(wv + stride), ld(wv + 2 * stride),
+                      sL[v * SC_THREADS + t], sR[v * SC_THREADS + t]);
+        }
+    }
+    __syncthreads();
+
+    // ---- phase B: Lax-Friedrichs flux of face m+1/2, stored over the left state
+    F2 Fv[9];
+    if (face) {
+        F2 uL[9], uR[9];
+#pragma unroll
+        for (int v = 0; v < 9; v++) uL[v] = sL[v * SC_THREADS + t], uR[v] = sR[v * SC_THREADS + t + STEP];
+        lf_flux<DIR>(n, lam, mu, buo, pk(0.5f * a.alpha), uL, uR, Fv);
+    } else {
+#pragma unroll
+        for (int v = 0; v < 9; v++) Fv[v] = pk(0.0f);
+    }
+#pragma unroll
+    for (int v = 0; v < 9; v++) sL[v * SC_THREADS + t] = Fv[v];
+    __syncthreads();
+
+    // ---- phase C: flux difference at the tile's points
+    if (!have || mi < 3 || mi > NPOS - 4 || m >= nd) return;
+    F2 val[9];
+    const F2 coef = ld(a.sjac + q);   // DT * rDH / J
+    if (k >= _nz - 3) {
+        for (int l = 0; l < (two ? 2 : 1); l++) {
+            float Fp[9], Fm[9], r[9], c[2];
+            unpk(coef, c[0], c[1]);
+            for (int v = 0; v < 9; v++) {
+                float x[2];
+                unpk(sL[v * SC_THREADS + t], x[0], x[1]);
+                Fp[v] = l ? x[1] : x[0];
+                unpk(sL[v * SC_THREADS + t - STEP], x[0], x[1]);
+                Fm[v] = l ? x[1] : x[0];
+            }
+            const long long ql = q + l * (DIR == 0 ? g.pitch : 1);
+            const int mc0 = DIR == 0 ? C_XI_X : DIR == 1 ? C_ET_X : C_ZT_X;
+            surface_diff(a, ql, stride, mc0, l ? c[1] : c[0], Fp, Fm, r);
+            epilogue<DIR>(a, ql, DIR == 0 ? i : i + l, DIR == 0 ? j + l : j, k, r);
+        }
+        return;
+    }
+    // faces p-5/2 .. p+5/2: the fourth- and sixth-order corrected flux is
+    // Fh = c2 F-2 + c1 F-1 + c0 F0 + c1 F+1 + c2 F+2 with c0 = 6402/5760,
+    // c1 = -348/5760, c2 = 27/5760; val = -coef (Fh[p] - Fh[p-1])
+    const F2 e0 = pk(27.0f / 5760) * coef, e1 = pk((-348.0f - 27.0f) / 5760) * coef,
+             e2 = pk((6402.0f + 348.0f) / 5760) * coef;
+#pragma unroll
+    for (int v = 0; v < 9; v++) {
+        const F2 *f = sL + v * SC_THREADS + t;
+        val[v] = fma2(e2, f[-STEP] - f[0], fma2(e1, f[-2 * STEP] - f[STEP], e0 * (f[-3 * STEP] - f[2 * STEP])));
+    }
+    epilogue2<DIR>(a, q, i, j, k, two, val);
+}
+#else
 template <int DIR, int NPOS, int NL>
 __global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const ScDirArgs a)
 {
@@ -366,7 +538,7 @@ __global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const 
             float uL[9], uR[9];
 #pragma unroll
             for (int v = 0; v < 9; v++) uL[v] = sL[sidx(v, mi, lane)], uR[v] = sR[sidx(v, mi + 1, lane)];
-            lf_flux(n0, n1, n2, lam, mu, buo, a.alpha, uL, uR, Fv);
+            lf_flux_ref(n0, n1, n2, lam, mu, buo, a.alpha, uL, uR, Fv);
         } else {
 #pragma unroll
             for (int v = 0; v < 9; v++) Fv[v] = 0.0f;
@@ -398,12 +570,13 @@ __global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const 
                 float f[6];
 #pragma unroll
                 for (int t = 0; t < 6; t++) f[t] = sL[sidx(v, pi + t, lane)];  // faces p-5/2 .. p+5/2
-                val[v] = interior_diff(f, coef);
+                val[v] = interior_diff_ref(f, coef);
             }
         }
         epilogue<DIR>(a, q, i, j, k, val);
     }
 }
+#endif
 
 // --------------------------------------------------------- free surface
 // One thread per surface column (src/freeSurface.cpp:40-194).  The

@@ -1,0 +1,49 @@
+"""ME-AWENO passes at the edges of their tiles: the default build (two points
+a thread) against the FP64 run of the same model.
+
+The x pass has tiles of 58 points x 8 rows, the y and z passes of 26 points x
+16 columns, taken in pairs of rows or columns, so sizes run over one tile, one
+point more, odd remainders and the smallest model the scheme accepts.  The
+bound is the distance the same algorithm in FP32 with every operation rounded
+keeps from FP64 (the exact build's), doubled.
+"""
+
+import numpy as np
+import pytest
+
+import parity_util as pu
+from cgfdm import Session, cases
+
+
+def _run(nx, ny, nz, source, tmp):
+    c = cases.halfspace_case(NX=nx, NY=ny, NZ=nz, nPML=5, steps=24, n_stations=3, depth_m=300.0, courant=0.4)
+    c.fault = []
+    c.gauss_hill = 1
+    at = (nx // 2, ny // 2, nz // 2)
+    if source == "ricker":
+        c.ricker_point = at + (8.0,)
+    else:
+        c.double_couple = dict(X=at[0], Y=at[1], Z=at[2], strike=40.0, dip=55.0, rake=70.0, Mw=8.0, duration=0.6)
+    c.stations = [(at[0], at[1], nz - 1), (at[0] - 3, at[1] + 3, nz // 2), (nx - 1, ny - 1, nz - 1)]
+    return cases.write_case(c, str(tmp / "run"), scheme="SCFDM")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nz,source", [(8, 7, 8, "couple"), (26, 26, 26, "ricker"), (27, 25, 27, "couple"),
+                                             (58, 16, 13, "couple"), (59, 17, 15, "ricker"), (33, 53, 9, "couple"),
+                                             (15, 9, 53, "couple")])
+def test_passes_match_fp64(tmp_path, nx, ny, nz, source):
+    d = _run(nx, ny, nz, source, tmp_path)
+    err = {}
+    with Session(d) as s:
+        st64, _, W64 = s.run_precise(24, bits=64, wavefield=True)
+    assert np.abs(W64[3:-3, 3:-3, 3:-3]).max() > 0
+    for flavor in ("fast", "exact"):
+        with Session(d, flavor=flavor) as s:
+            s.run(24)
+            W, st = s.wavefield(), s.stations()
+        # momentum and strain have their own scales; halo layers are compared too
+        err[flavor] = max(pu.rel_l2(W[..., :3], W64[..., :3]), pu.rel_l2(W[..., 3:], W64[..., 3:]),
+                          pu.rel_l2(st[..., :3], st64[..., :3]), pu.rel_l2(st[..., 3:], st64[..., 3:]))
+    print(f"{nx}x{ny}x{nz} {source}: fast {err['fast']:.2e}, exact {err['exact']:.2e}")
+    assert err["fast"] <= 2 * err["exact"] + 1e-7
