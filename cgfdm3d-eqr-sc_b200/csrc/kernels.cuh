@@ -200,8 +200,19 @@ struct ScTiling {
 };
 ScTiling sc_tiling(const DevGrid &g);
 
-cudaError_t sc_dir_prepare();
-cudaError_t launch_sc_dir(int dir, ScDirArgs a, const ScTiling &t, cudaStream_t st);
+// One launch of a pass: the tensor map of its input with the pass's box (128
+// bytes, from sc_tmap), the tiles in walking order (n0 fastest) and the
+// device error word (bit 0: a bounded wait for a copy gave up, bit 1: the
+// drain after it did).
+struct alignas(64) ScPass {
+    unsigned char tm[128];
+    ScDirArgs a;
+    int n0, n1, n2, total;
+    int *err;
+};
+cudaError_t sc_tmap(void *out, const float *base, const DevGrid &g, int dir);
+cudaError_t launch_sc_dir(int dir, const ScDirArgs &a, const ScTiling &t, const unsigned char *tmap, int *err, int sms,
+                          cudaStream_t st);
 // Characteristic free surface, halo extrapolation, sponge of the top layers,
 // peak ground velocity and (dis given) the surface-layer displacement, after
 // the third stage of a step.

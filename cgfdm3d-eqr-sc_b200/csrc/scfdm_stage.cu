@@ -40,10 +40,14 @@
 // smoothness indicators between the two states of a position, combines the
 // two fluxes of a face before applying the (linear) flux function, and folds
 // the flux-difference corrections into one six-tap filter.
+#include <algorithm>
+#include <cstring>
+
 #include "device.cuh"
 #include "kernels.cuh"
 #include "pair.cuh"
 #include "sc_ops.cuh"
+#include "tma.cuh"
 
 // 1: the passes' RHS and stage-output stores evict-first (each is read back
 // by a later pass or stage, long after L2 has turned over)
@@ -183,6 +187,7 @@ __device__ __forceinline__ float decay_apply(float w, int i, int j, int k, const
 
 }  // namespace
 
+#ifdef CGFDM_EXACT
 // Flux difference of one point in the top three layers: the corrections
 // come from point fluxes at p-3 .. p+3 along the direction
 // (src/alternative_flux_FD.cpp:1253-1279).  Fp, Fm: fluxes of the faces
@@ -231,6 +236,7 @@ __device__ __noinline__ void surface_diff(const ScDirArgs &a, long long q, long 
         val[v] = coef * (-(A - B));
     }
 }
+#endif
 
 // The pass's use of the flux difference val of point q = (i, j, k): the x
 // pass stores the RHS, the y pass adds to it, the z pass adds its part and
@@ -238,6 +244,7 @@ __device__ __noinline__ void surface_diff(const ScDirArgs &a, long long q, long 
 // the top four layers in the last stage, and carries the halo above the
 // surface into the stage buffer in stages 0 and 1 (the reference's update
 // runs over every point; halo points have a zero RHS and keep their value).
+#ifdef CGFDM_EXACT
 template <int DIR>
 __device__ __forceinline__ void epilogue(const ScDirArgs &a, long long q, int i, int j, int k, const float val[9])
 {
@@ -275,68 +282,121 @@ __device__ __forceinline__ void epilogue(const ScDirArgs &a, long long q, int i,
                 for (int v = 0; v < 9; v++) a.Wout[v * F + q + h * a.g.plane] = a.W[v * F + q + h * a.g.plane];
     }
 }
-
-#ifndef CGFDM_EXACT
-// The same for two neighbouring points (rows j, j+1 of the x pass, columns
-// i, i+1 of the others); two: the second one is inside the grid.
+#else
+// Two neighbouring points at once (rows j, j+1 of the x pass, columns i, i+1
+// of the others); two: the second one is inside the grid.  val is the
+// RHS so far with this pass's part, w0 the stage input.
 template <int DIR>
 __device__ __forceinline__ void epilogue2(const ScDirArgs &a, long long q, int i, int j, int k, bool two,
-                                          const F2 val[9])
+                                          const F2 val[9], const F2 w0[9])
 {
     const long long F = a.g.fstride;
-    auto ld = [&](const float *p) { return SC_LD(*reinterpret_cast<const float2 *>(p)); };
-    auto st = [&](float *p, float x, float y) {
-        if (two) SC_ST(*reinterpret_cast<float2 *>(p), make_float2(x, y));
+    auto st = [&](float *p, F2 v) {
+        float x, y;
+        unpk(v, x, y);
+        if (DIR == 0) {
+            SC_ST(*p, x);
+            if (two) SC_ST(p[a.g.pitch], y);
+        } else if (two) SC_ST(*reinterpret_cast<float2 *>(p), make_float2(x, y));
         else SC_ST(*p, x);
     };
-    if (DIR == 0) {
+    if (DIR < 2) {
 #pragma unroll
-        for (int v = 0; v < 9; v++) {
+        for (int v = 0; v < 9; v++) st(a.H + v * F + q, val[v]);
+        return;
+    }
+    const int _nz = a.g.nzp - CGFDM_HALO;
+    const bool decay = a.decay != nullptr && k < _nz - 4;
+    auto rk = [&](float m, float w, float h) -> float {
+        if (a.irk == 1)
+            return __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(0.75, (double)m), __dmul_rn(0.25, (double)w)),
+                                               __dmul_rn(0.25, (double)h)));
+        return __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(1.0 / 3.0, (double)m), __dmul_rn(2.0 / 3.0, (double)w)),
+                                           __dmul_rn(2.0 / 3.0, (double)h)));
+    };
+    float2 m[9];
+    if (a.irk != 0)
+#pragma unroll
+        for (int v = 0; v < 9; v++) m[v] = SC_LD(*reinterpret_cast<const float2 *>(a.Wm + v * F + q));
+#pragma unroll
+    for (int v = 0; v < 9; v++) {
+        F2 o;
+        if (a.irk == 0) o = w0[v] + val[v];
+        else {
+            float wx, wy, hx, hy;
+            unpk(w0[v], wx, wy);
+            unpk(val[v], hx, hy);
+            o = pk(rk(m[v].x, wx, hx), rk(m[v].y, wy, hy));
+        }
+        if (decay) {
             float x, y;
-            unpk(val[v], x, y);
-            SC_ST(a.H[v * F + q], x);
-            if (two) SC_ST(a.H[v * F + q + a.g.pitch], y);
+            unpk(o, x, y);
+            o = pk(decay_apply(x, i, j, k, a.g, a.decay, a.ndecay), decay_apply(y, i + 1, j, k, a.g, a.decay, a.ndecay));
         }
-    } else if (DIR == 1) {
-        F2 h[9];
+        st(a.Wout + v * F + q, o);
+    }
+    if (a.copy_halo && k == _nz - 1)
+#pragma unroll 1
+        for (int h = 1; h <= CGFDM_HALO; h++)
 #pragma unroll
-        for (int v = 0; v < 9; v++) {
-            const float2 w = ld(a.H + v * F + q);
-            h[v] = pk(w.x, w.y) + val[v];
-        }
-#pragma unroll
-        for (int v = 0; v < 9; v++) {
-            float x, y;
-            unpk(h[v], x, y);
-            st(a.H + v * F + q, x, y);
-        }
-    } else {
-        const int _nz = a.g.nzp - CGFDM_HALO;
-        const bool decay = a.decay != nullptr && k < _nz - 4;
-        auto rk = [&](float m, float w, float h) -> float {
-            if (a.irk == 1)
-                return __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(0.75, (double)m), __dmul_rn(0.25, (double)w)),
-                                                   __dmul_rn(0.25, (double)h)));
-            return __double2float_rn(__dadd_rn(__dadd_rn(__dmul_rn(1.0 / 3.0, (double)m),
-                                                         __dmul_rn(2.0 / 3.0, (double)w)),
-                                               __dmul_rn(2.0 / 3.0, (double)h)));
-        };
-#pragma unroll 3
-        for (int v = 0; v < 9; v++) {
-            const float2 h0 = ld(a.H + v * F + q), w = *reinterpret_cast<const float2 *>(a.W + v * F + q);
-            float2 m = make_float2(0.0f, 0.0f), o;
-            if (a.irk != 0) m = ld(a.Wm + v * F + q);
-            float hx, hy;
-            unpk(pk(h0.x, h0.y) + val[v], hx, hy);
-            if (a.irk == 0) o.x = w.x + hx, o.y = w.y + hy;
-            else o.x = rk(m.x, w.x, hx), o.y = rk(m.y, w.y, hy);
-            if (decay) {
-                o.x = decay_apply(o.x, i, j, k, a.g, a.decay, a.ndecay);
-                o.y = decay_apply(o.y, i + 1, j, k, a.g, a.decay, a.ndecay);
+            for (int v = 0; v < 9; v++) {
+                const long long e = v * F + q + h * a.g.plane;
+                const float2 w = *reinterpret_cast<const float2 *>(a.W + e);
+                st(a.Wout + e, pk(w.x, w.y));
             }
-            st(a.Wout + v * F + q, o.x, o.y);
+}
+
+// Flux difference val of two points in the top three layers, where the
+// corrections come from point fluxes hu at p-3 .. p+3 along the direction
+// (src/alternative_flux_FD.cpp:1253-1279).  With both faces' second and
+// fourth differences collected,
+//   val = -coef (Fp - Fm + (57 (hu[3] - hu[-3]) - 468 (hu[2] - hu[-2]) + 765 (hu[1] - hu[-1])) / 11520),
+// Fp, Fm the fluxes of the faces p+1/2 and p-1/2: six linear fluxes summed
+// into nine registers.  (Point by point with the reference's four sums of
+// nine, the one warp of a z tile that holds the top layers kept the other
+// seven waiting: 5.7 of 18.5 cycles an instruction at the barrier.)
+template <int DIR, class LD>
+__device__ __forceinline__ void surface_diff(const ScDirArgs &a, long long q, long long stride, F2 coef, const F2 *Fp,
+                                             const F2 *Fm, LD ld, F2 val[9])
+{
+    const long long F = a.g.fstride;
+    constexpr float w[6] = {-57.0f / 11520, 468.0f / 11520, -765.0f / 11520, 765.0f / 11520, -468.0f / 11520,
+                            57.0f / 11520};
+#pragma unroll
+    for (int v = 0; v < 9; v++) val[v] = Fm[v * SC_THREADS] - Fp[v * SC_THREADS];
+#pragma unroll 1
+    for (int t = 0; t < 6; t++) {
+        const long long qn = q + (t < 3 ? t - 3 : t - 2) * stride;
+        const float *c = a.cjm + qn, *u = a.W + qn;
+        const F2 lam = ld(c + C_LAMBDA * F), mu = ld(c + C_MU * F), buo = ld(c + C_BUOY * F), s = pk(w[t]);
+        const F2 u0 = ld(u), u1 = ld(u + F), u2 = ld(u + 2 * F), u3 = ld(u + 3 * F), u4 = ld(u + 4 * F),
+                 u5 = ld(u + 5 * F), u6 = ld(u + 6 * F), u7 = ld(u + 7 * F), u8 = ld(u + 8 * F);
+        const F2 ltr = lam * ((u3 + u4) + u5), m2 = mu + mu;
+        // -hu, the flux without its sign, times s
+        if constexpr (DIR == 0) {
+            const F2 n = s * ld(c + C_XI_X * F), nm = n * mu, nb = n * buo;
+            val[0] = fma2(n, fma2(m2, u3, ltr), val[0]);
+            val[1] = fma2(nm, u8, val[1]), val[2] = fma2(nm, u7, val[2]);
+            val[3] = fma2(nb, u0, val[3]), val[7] = fma2(nb, u2, val[7]), val[8] = fma2(nb, u1, val[8]);
+        } else if constexpr (DIR == 1) {
+            const F2 n = s * ld(c + C_ET_Y * F), nm = n * mu, nb = n * buo;
+            val[1] = fma2(n, fma2(m2, u4, ltr), val[1]);
+            val[0] = fma2(nm, u8, val[0]), val[2] = fma2(nm, u6, val[2]);
+            val[4] = fma2(nb, u1, val[4]), val[6] = fma2(nb, u2, val[6]), val[8] = fma2(nb, u0, val[8]);
+        } else {
+            const F2 n0 = s * ld(c + C_ZT_X * F), n1 = s * ld(c + C_ZT_Y * F), n2 = s * ld(c + C_ZT_Z * F);
+            const F2 m0 = n0 * mu, m1 = n1 * mu, mm = n2 * mu, b0 = n0 * buo, b1 = n1 * buo, b2 = n2 * buo;
+            val[0] = fma2(n0, fma2(m2, u3, ltr), fma2(m1, u8, fma2(mm, u7, val[0])));
+            val[1] = fma2(n1, fma2(m2, u4, ltr), fma2(m0, u8, fma2(mm, u6, val[1])));
+            val[2] = fma2(n2, fma2(m2, u5, ltr), fma2(m0, u7, fma2(m1, u6, val[2])));
+            val[3] = fma2(b0, u0, val[3]), val[4] = fma2(b1, u1, val[4]), val[5] = fma2(b2, u2, val[5]);
+            val[6] = fma2(b1, u2, fma2(b2, u1, val[6]));
+            val[7] = fma2(b0, u2, fma2(b2, u0, val[7]));
+            val[8] = fma2(b0, u1, fma2(b1, u0, val[8]));
         }
     }
+#pragma unroll
+    for (int v = 0; v < 9; v++) val[v] = coef * val[v];
 }
 #endif
 
@@ -360,112 +420,188 @@ constexpr int SCX_NPOS = 64, SCX_NL = 8;
 constexpr int SCX_NPOS = 64, SCX_NL = 4;
 #endif
 constexpr int SCY_NPOS = 32, SCY_NL = 16;
+// two CTAs an SM: the 128 registers hold the epilogue's operands over a
+// barrier (three at 80 registers, loading them after it: 17.1 against 14.9 ms
+// per step on 384 x 384 x 192)
 #ifndef SC_TILE_MIN_CTAS
-#define SC_TILE_MIN_CTAS 3
+#define SC_TILE_MIN_CTAS 2
 #endif
 // shared memory of a tile: left and right states, 9 + 9 fields per position
 constexpr size_t sc_tile_smem(int npos, int nl) { return sizeof(float) * 18 * npos * nl; }
 
 #ifndef CGFDM_EXACT
+// The box of W a tile's states need, two more positions on either side: 72 x
+// 8 rows (from a 16-byte boundary, so up to three columns early) for the x
+// pass, 16 x 36 for the others; both 20736 bytes for the nine fields.
+constexpr int SC_BOX_F = 36 * 16 * 9;
+static_assert(SC_BOX_F == 72 * 8 * 9 && SC_BOX_F * 4 % 128 == 0, "one box size for the three passes");
+constexpr size_t SC_PASS_SMEM = sizeof(float) * (SC_BOX_F + 2 * 18 * SC_THREADS) + 8;
+
+// Persistent CTAs, two on an SM, walk the tiles in order.  A tile's box of
+// W arrives by TMA while the tile before it is in phases B and C, and the
+// values its epilogue adds to are loaded before the barrier that ends phase
+// B, so the passes no longer wait for memory in every phase (with plain loads
+// the z pass spent 7 of 12 cycles an instruction on them).
 template <int DIR, int NPOS, int NL>
-__global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const ScDirArgs a)
+__global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const __grid_constant__ ScPass p)
 {
     constexpr int PR = NL / 2;                     // lane pairs
     constexpr int STEP = DIR == 0 ? 1 : PR;        // threads from one position to the next
     static_assert(NPOS * PR == SC_THREADS, "one position of one lane pair a thread");
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    F2 *sL = reinterpret_cast<F2 *>(sm_raw), *sR = sL + 9 * SC_THREADS;
+    extern __shared__ __align__(128) unsigned char sm_raw[];
+    float *sW = reinterpret_cast<float *>(sm_raw);
+    F2 *sL = reinterpret_cast<F2 *>(sm_raw + SC_BOX_F * 4), *sR = sL + 9 * SC_THREADS;
+    const unsigned bar = smem_u32(sR + 9 * SC_THREADS);
+    const ScDirArgs &a = p.a;
     const DevGrid &g = a.g;
     const long long F = g.fstride;
     const int _nx = g.nxp - CGFDM_HALO, _ny = g.nyp - CGFDM_HALO, _nz = g.nzp - CGFDM_HALO;
     const int nd = DIR == 0 ? _nx : DIR == 1 ? _ny : _nz;  // points along the pass end before nd
     const long long stride = DIR == 0 ? 1 : DIR == 1 ? (long long)g.pitch : g.plane;
-    const int tile = DIR == 0 ? blockIdx.x : DIR == 1 ? blockIdx.y : blockIdx.z;
     const int lane_end = DIR == 0 ? _ny : _nx;
     const int t = threadIdx.x;
     const int mi = DIR == 0 ? t % NPOS : t / PR, pr = DIR == 0 ? t / NPOS : t % PR;
-    const int m = tile * (NPOS - 6) + mi;                                           // padded index along the pass
-    const int lane = CGFDM_HALO + (DIR == 0 ? blockIdx.y : blockIdx.x) * NL + 2 * pr;
-    const int i = DIR == 0 ? m : lane, j = DIR == 0 ? lane : DIR == 1 ? m : CGFDM_HALO + (int)blockIdx.y,
-              k = DIR == 2 ? m : CGFDM_HALO + (int)blockIdx.z;
-    // the pair's second lane may be the first halo lane of a row (read, never
-    // written); columns lie on 8-byte boundaries (xoff 1, tiles of 16)
-    const bool have = lane < lane_end, two = lane + 1 < lane_end;
-    const long long q = g.at(i, j, k);
-    auto ld = [&](const float *p) -> F2 {
-        if constexpr (DIR == 0) return pk(__ldg(p), __ldg(p + g.pitch));
-        else {
-            const float2 w = __ldg(reinterpret_cast<const float2 *>(p));
-            return pk(w.x, w.y);
-        }
+    // tile u: its number along the pass, lane group and plane (row for the z pass)
+    auto split = [&](int u, int &tile, int &group, int &rest) {
+        const int x = u % p.n0, y = u / p.n0 % p.n1, z = u / p.n0 / p.n1;
+        if (DIR == 0) tile = x, group = y, rest = z;
+        else if (DIR == 1) group = x, tile = y, rest = z;
+        else group = x, rest = y, tile = z;
     };
-    // ---- phase A: both WENO states of every position
-    const bool face = have && mi < NPOS - 1 && m >= 2 && m < nd;
-    F2 n[3], lam, mu, buo;
-    if (face) {
-        if constexpr (DIR < 2) n[0] = ld(a.cjm + (DIR == 0 ? C_XI_X : C_ET_Y) * F + q);
-        else n[0] = ld(a.cjm + C_ZT_X * F + q), n[1] = ld(a.cjm + C_ZT_Y * F + q), n[2] = ld(a.cjm + C_ZT_Z * F + q);
-        lam = ld(a.cjm + C_LAMBDA * F + q), mu = ld(a.cjm + C_MU * F + q), buo = ld(a.cjm + C_BUOY * F + q);
-    }
-    if (have && m >= 2 && m <= nd) {
-        const float *w = a.W + q;
-#pragma unroll 3
-        for (int v = 0; v < 9; v++) {
-            const float *wv = w + v * F;
-            weno_pair(ld(wv - 2 * stride), ld(wv - stride), ld(wv), ld(wv + stride), ld(wv + 2 * stride),
-                      sL[v * SC_THREADS + t], sR[v * SC_THREADS + t]);
-        }
+    auto issue = [&](int u) {
+        int tile, group, rest;
+        split(u, tile, group, rest);
+        const int m0 = tile * (NPOS - 6) - 2, l0 = CGFDM_HALO + group * NL, r = CGFDM_HALO + rest;
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        mbar_expect_tx(bar, SC_BOX_F * 4);
+        if (DIR == 0) tma_load_4d(smem_u32(sW), p.tm, (g.xoff + m0) & ~3, l0, r, 0, bar);
+        else if (DIR == 1) tma_load_4d(smem_u32(sW), p.tm, g.xoff + l0, m0, r, 0, bar);
+        else tma_load_4d(smem_u32(sW), p.tm, g.xoff + l0, r, m0, 0, bar);
+    };
+    if (t == 0) {
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        issue(blockIdx.x);                         // the grid has no more CTAs than tiles
     }
     __syncthreads();
-
-    // ---- phase B: Lax-Friedrichs flux of face m+1/2, stored over the left state
-    F2 Fv[9];
-    if (face) {
-        F2 uL[9], uR[9];
-#pragma unroll
-        for (int v = 0; v < 9; v++) uL[v] = sL[v * SC_THREADS + t], uR[v] = sR[v * SC_THREADS + t + STEP];
-        lf_flux<DIR>(n, lam, mu, buo, pk(0.5f * a.alpha), uL, uR, Fv);
-    } else {
-#pragma unroll
-        for (int v = 0; v < 9; v++) Fv[v] = pk(0.0f);
-    }
-#pragma unroll
-    for (int v = 0; v < 9; v++) sL[v * SC_THREADS + t] = Fv[v];
-    __syncthreads();
-
-    // ---- phase C: flux difference at the tile's points
-    if (!have || mi < 3 || mi > NPOS - 4 || m >= nd) return;
-    F2 val[9];
-    const F2 coef = ld(a.sjac + q);   // DT * rDH / J
-    if (k >= _nz - 3) {
-        for (int l = 0; l < (two ? 2 : 1); l++) {
-            float Fp[9], Fm[9], r[9], c[2];
-            unpk(coef, c[0], c[1]);
-            for (int v = 0; v < 9; v++) {
-                float x[2];
-                unpk(sL[v * SC_THREADS + t], x[0], x[1]);
-                Fp[v] = l ? x[1] : x[0];
-                unpk(sL[v * SC_THREADS + t - STEP], x[0], x[1]);
-                Fm[v] = l ? x[1] : x[0];
+    unsigned phase = 0;
+#pragma unroll 1
+    for (int u = blockIdx.x; u < p.total; u += gridDim.x, phase ^= 1) {
+        int tile, group, rest;
+        split(u, tile, group, rest);
+        const int m = tile * (NPOS - 6) + mi;                                       // padded index along the pass
+        const int lane = CGFDM_HALO + group * NL + 2 * pr;
+        const int i = DIR == 0 ? m : lane, j = DIR == 0 ? lane : DIR == 1 ? m : CGFDM_HALO + rest,
+                  k = DIR == 2 ? m : CGFDM_HALO + rest;
+        // the pair's second lane may be the first halo lane of a row (read, never
+        // written); columns lie on 8-byte boundaries (xoff 1, tiles of 16)
+        const bool have = lane < lane_end, two = lane + 1 < lane_end;
+        const long long q = g.at(i, j, k);
+        auto ld = [&](const float *x) -> F2 {
+            if constexpr (DIR == 0) return pk(__ldg(x), __ldg(x + g.pitch));
+            else {
+                const float2 w = __ldg(reinterpret_cast<const float2 *>(x));
+                return pk(w.x, w.y);
             }
-            const long long ql = q + l * (DIR == 0 ? g.pitch : 1);
-            const int mc0 = DIR == 0 ? C_XI_X : DIR == 1 ? C_ET_X : C_ZT_X;
-            surface_diff(a, ql, stride, mc0, l ? c[1] : c[0], Fp, Fm, r);
-            epilogue<DIR>(a, ql, DIR == 0 ? i : i + l, DIR == 0 ? j + l : j, k, r);
+        };
+        const bool face = have && mi < NPOS - 1 && m >= 2 && m < nd;
+        const bool point = have && mi >= 3 && mi <= NPOS - 4 && m < nd;
+        // ---- phase A: both WENO states of every position
+        const bool ok = mbar_wait_bounded(bar, phase, 1LL << 31);
+        if (ok && have && m >= 2 && m <= nd) {
+            // this position's value in the box, the next field SF and the next position SP floats on
+            constexpr int SF = DIR == 0 ? 72 * NL : 36 * NL, SP = DIR == 0 ? 1 : NL;
+            const float *w = DIR == 0 ? sW + 2 * pr * 72 + ((g.xoff + tile * (NPOS - 6) - 2) & 3) + mi + 2
+                                      : sW + (mi + 2) * NL + 2 * pr;
+            auto at = [&](int v, int o) -> F2 {
+                const float *x = w + v * SF + o * SP;
+                if constexpr (DIR == 0) return pk(x[0], x[72]);
+                else {
+                    const float2 y = *reinterpret_cast<const float2 *>(x);
+                    return pk(y.x, y.y);
+                }
+            };
+#pragma unroll 3
+            for (int v = 0; v < 9; v++)
+                weno_pair(at(v, -2), at(v, -1), at(v, 0), at(v, 1), at(v, 2), sL[v * SC_THREADS + t],
+                          sR[v * SC_THREADS + t]);
         }
-        return;
-    }
-    // faces p-5/2 .. p+5/2: the fourth- and sixth-order corrected flux is
-    // Fh = c2 F-2 + c1 F-1 + c0 F0 + c1 F+1 + c2 F+2 with c0 = 6402/5760,
-    // c1 = -348/5760, c2 = 27/5760; val = -coef (Fh[p] - Fh[p-1])
-    const F2 e0 = pk(27.0f / 5760) * coef, e1 = pk((-348.0f - 27.0f) / 5760) * coef,
-             e2 = pk((6402.0f + 348.0f) / 5760) * coef;
+        // (in flight over the barrier)
+        F2 n[3], lam, mu, buo;
+        if (face) {
+            if constexpr (DIR < 2) n[0] = ld(a.cjm + (DIR == 0 ? C_XI_X : C_ET_Y) * F + q);
+            else n[0] = ld(a.cjm + C_ZT_X * F + q), n[1] = ld(a.cjm + C_ZT_Y * F + q), n[2] = ld(a.cjm + C_ZT_Z * F + q);
+            lam = ld(a.cjm + C_LAMBDA * F + q), mu = ld(a.cjm + C_MU * F + q), buo = ld(a.cjm + C_BUOY * F + q);
+        }
+        if (__syncthreads_or(!ok)) {
+            // a copy that did not arrive: nothing more is computed, and no copy
+            // may still be landing in shared memory when the CTA exits
+            if (t == 0) {
+                atomicOr(p.err, 1);
+                if (!mbar_wait_bounded(bar, phase, 1LL << 31)) atomicOr(p.err, 2);
+            }
+            __syncthreads();
+            return;
+        }
+        if (t == 0 && u + (int)gridDim.x < p.total) issue(u + gridDim.x);
+
+        // ---- phase B: Lax-Friedrichs flux of face m+1/2, stored over the left state
+        {
+            F2 Fv[9];
+            if (face) {
+                F2 uL[9], uR[9];
 #pragma unroll
-    for (int v = 0; v < 9; v++) {
-        const F2 *f = sL + v * SC_THREADS + t;
-        val[v] = fma2(e2, f[-STEP] - f[0], fma2(e1, f[-2 * STEP] - f[STEP], e0 * (f[-3 * STEP] - f[2 * STEP])));
+                for (int v = 0; v < 9; v++) uL[v] = sL[v * SC_THREADS + t], uR[v] = sR[v * SC_THREADS + t + STEP];
+                lf_flux<DIR>(n, lam, mu, buo, pk(0.5f * a.alpha), uL, uR, Fv);
+            } else {
+#pragma unroll
+                for (int v = 0; v < 9; v++) Fv[v] = pk(0.0f);
+            }
+#pragma unroll
+            for (int v = 0; v < 9; v++) sL[v * SC_THREADS + t] = Fv[v];
+        }
+        F2 h[9], w0[9], coef;
+        if (point) {
+            coef = ld(a.sjac + q);   // DT * rDH / J
+#pragma unroll
+            for (int v = 0; v < 9; v++) {
+                if (DIR > 0) {
+                    const float2 x = SC_LD(*reinterpret_cast<const float2 *>(a.H + v * F + q));
+                    h[v] = pk(x.x, x.y);
+                }
+                if (DIR == 2) {
+                    const float2 x = *reinterpret_cast<const float2 *>(a.W + v * F + q);
+                    w0[v] = pk(x.x, x.y);
+                }
+            }
+        }
+        __syncthreads();
+
+        // ---- phase C: flux difference at the tile's points
+        if (point) {
+            F2 val[9];
+            if (k >= _nz - 3) {
+                surface_diff<DIR>(a, q, stride, coef, sL + t, sL + t - STEP, ld, val);
+            } else {
+                // faces p-5/2 .. p+5/2: the fourth- and sixth-order corrected flux is
+                // Fh = c2 F-2 + c1 F-1 + c0 F0 + c1 F+1 + c2 F+2 with c0 = 6402/5760,
+                // c1 = -348/5760, c2 = 27/5760; val = -coef (Fh[p] - Fh[p-1])
+                const F2 e0 = pk(27.0f / 5760) * coef, e1 = pk((-348.0f - 27.0f) / 5760) * coef,
+                         e2 = pk((6402.0f + 348.0f) / 5760) * coef;
+#pragma unroll
+                for (int v = 0; v < 9; v++) {
+                    const F2 *f = sL + v * SC_THREADS + t;
+                    val[v] = fma2(e2, f[-STEP] - f[0],
+                                  fma2(e1, f[-2 * STEP] - f[STEP], e0 * (f[-3 * STEP] - f[2 * STEP])));
+                }
+            }
+            if (DIR > 0)
+#pragma unroll
+                for (int v = 0; v < 9; v++) val[v] = h[v] + val[v];
+            epilogue2<DIR>(a, q, i, j, k, two, val, w0);
+        }
+        __syncthreads();                           // the fluxes are read: the next tile's states may overwrite them
     }
-    epilogue2<DIR>(a, q, i, j, k, two, val);
 }
 #else
 template <int DIR, int NPOS, int NL>
@@ -665,22 +801,55 @@ ScTiling sc_tiling(const DevGrid &g)
     return t;
 }
 
+#ifndef CGFDM_EXACT
+// The tensor map of a nine-field buffer with the box of pass dir.
+cudaError_t sc_tmap(void *out, const float *base, const DevGrid &g, int dir)
+{
+    const auto encode = tmap_encoder();
+    if (!encode) return cudaErrorNotSupported;
+    cuuint64_t dims[4] = {(cuuint64_t)g.pitch, (cuuint64_t)g.nyp, (cuuint64_t)g.nzp, 9};
+    cuuint64_t strides[3] = {(cuuint64_t)g.pitch * 4, (cuuint64_t)g.plane * 4, (cuuint64_t)g.fstride * 4};
+    cuuint32_t box[4] = {dir == 0 ? 72u : (cuuint32_t)SCY_NL, dir == 0 ? (cuuint32_t)SCX_NL : dir == 1 ? 36u : 1u,
+                         dir == 2 ? 36u : 1u, 9};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = encode(reinterpret_cast<CUtensorMap *>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)base,
+                              dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 template <int DIR, int NPOS, int NL>
-static cudaError_t tile_attr()
+static cudaError_t launch_pass(ScPass &p, int sms, cudaStream_t st)
 {
-    return cudaFuncSetAttribute(k_sc_tile<DIR, NPOS, NL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sc_tile_smem(NPOS, NL));
+    CUDA_TRY(cudaFuncSetAttribute(k_sc_tile<DIR, NPOS, NL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)SC_PASS_SMEM));
+    p.total = p.n0 * p.n1 * p.n2;
+    const int grid = std::min(p.total, sms * SC_TILE_MIN_CTAS);
+    k_sc_tile<DIR, NPOS, NL><<<grid, SC_THREADS, SC_PASS_SMEM, st>>>(p);
+    return cudaGetLastError();
 }
 
-cudaError_t sc_dir_prepare()
+cudaError_t launch_sc_dir(int dir, const ScDirArgs &a, const ScTiling &t, const unsigned char *tmap, int *err, int sms,
+                          cudaStream_t st)
 {
-    CUDA_TRY((tile_attr<0, SCX_NPOS, SCX_NL>()));
-    CUDA_TRY((tile_attr<1, SCY_NPOS, SCY_NL>()));
-    CUDA_TRY((tile_attr<2, SCY_NPOS, SCY_NL>()));
-    return cudaSuccess;
+    const DevGrid &g = a.g;
+    ScPass p{};
+    std::memcpy(p.tm, tmap, sizeof p.tm);
+    p.a = a;
+    p.err = err;
+    const int along = t.ntiles[dir], groups = ((dir == 0 ? g.ny : g.nx) + t.nl[dir] - 1) / t.nl[dir];
+    if (dir == 0) {
+        p.n0 = along, p.n1 = groups, p.n2 = g.nz;
+        return launch_pass<0, SCX_NPOS, SCX_NL>(p, sms, st);
+    }
+    p.n0 = groups, p.n1 = dir == 1 ? along : g.ny, p.n2 = dir == 1 ? g.nz : along;
+    return dir == 1 ? launch_pass<1, SCY_NPOS, SCY_NL>(p, sms, st) : launch_pass<2, SCY_NPOS, SCY_NL>(p, sms, st);
 }
+#else
+cudaError_t sc_tmap(void *, const float *, const DevGrid &, int) { return cudaSuccess; }   // plain loads
 
-cudaError_t launch_sc_dir(int dir, ScDirArgs a, const ScTiling &t, cudaStream_t st)
+cudaError_t launch_sc_dir(int dir, const ScDirArgs &a, const ScTiling &t, const unsigned char *, int *, int,
+                          cudaStream_t st)
 {
     const DevGrid &g = a.g;
     if (dir == 0) {
@@ -698,6 +867,7 @@ cudaError_t launch_sc_dir(int dir, ScDirArgs a, const ScTiling &t, cudaStream_t 
     }
     return cudaGetLastError();
 }
+#endif
 
 cudaError_t launch_sc_surface(float *W, const float *cjm, DevGrid g, const float *decayG, int ndecay, float *pgv,
                               float *dis, float DT, cudaStream_t st)

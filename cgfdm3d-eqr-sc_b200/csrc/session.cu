@@ -389,8 +389,11 @@ int Session::setup_device()
         ALLOC(h_, float, F * 9);
         ALLOC(sjac_, float, F);
         CU(launch_sc_sjac(cjm_, g, (float)m.p.DT, m.g.rDH, sjac_, stream));
-        CU(sc_dir_prepare());
         sct_ = sc_tiling(g);
+        for (int b = 0; b < 3; b++)
+            for (int dir = 0; dir < 3; dir++) CU(sc_tmap(sc_maps_[b][dir], W_[b], g, dir));
+        sms_ = 148;
+        cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device);
         if (m.p.exp_decay) {
             // G[p] = exp(-(alpha p)^2), p = 0 .. 20, in float as
             // src/exp_decay_absorb.cpp:45,110-111 evaluates it
@@ -759,7 +762,8 @@ int Session::launch_step(int step, bool timed_stages)
             a.copy_halo = irk < 2;
             a.alpha = m.Vp_max;
             if (timed_stages) CU(cudaEventRecord(ev_[2], stream));
-            for (int dir = 0; dir < 3; dir++) CU(launch_sc_dir(dir, a, sct_, stream));
+            for (int dir = 0; dir < 3; dir++)
+                CU(launch_sc_dir(dir, a, sct_, sc_maps_[irk][dir], err_dev_, sms_, stream));
             if (timed_stages) {
                 CU(cudaEventRecord(ev_[3], stream));
                 CU(cudaEventSynchronize(ev_[3]));

@@ -164,6 +164,8 @@ private:
     int *err_dev_ = nullptr;                         // device error word of the stage kernels
     float *h_ = nullptr, *sjac_ = nullptr, *decay_ = nullptr;  // SCFDM RHS, DT*rDH/J, sponge factors
     ScTiling sct_ = {};
+    alignas(64) unsigned char sc_maps_[3][3][128] = {};   // tensor maps of A, B, C for each pass
+    int sms_ = 148;
     static constexpr int SC_DECAY_LAYERS = 20;       // src/exp_decay_absorb.cpp:109
     int check_device_error();
     template <class R>
