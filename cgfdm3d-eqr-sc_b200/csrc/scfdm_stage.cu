@@ -78,12 +78,16 @@ __device__ __forceinline__ F2 operator+(F2 a, F2 b) { return vadd(a, b); }
 __device__ __forceinline__ F2 operator-(F2 a, F2 b) { return vsub(a, b); }
 __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return vmul(a, b); }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return vfma(a, b, c); }
+// (ftz: one instruction where the subnormal-safe form takes a compare, a
+// select and two multiplications; the arguments are squared indicators of at
+// least 8e-13 and sums of their reciprocals, subnormal only for differences
+// beyond 2e9 between neighbouring cells)
 __device__ __forceinline__ F2 rcp2(F2 x)
 {
     float a, b;
     unpk(x, a, b);
-    asm("rcp.approx.f32 %0, %0;" : "+f"(a));
-    asm("rcp.approx.f32 %0, %0;" : "+f"(b));
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(a));
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(b));
     return pk(a, b);
 }
 
