@@ -54,6 +54,17 @@
 #ifndef CG_PREFETCH_DIST
 #define CG_PREFETCH_DIST 1
 #endif
+// RK4 without the running sum: the step ends from the step start and the
+// three stage values, m + ((B - m) + 2 (C - m) + (D - m)) / 3 + h3 / 6, each in
+// a buffer of its own.  A step then moves 149 floats a point instead of 176
+// and 117 an absorbing-layer point instead of 144, and rounds less (the
+// differences are exact where the stages are close).  The exact build keeps
+// the reference's running sum T.
+#ifdef CGFDM_EXACT
+#define CG_RK_SUM 1
+#else
+#define CG_RK_SUM 0
+#endif
 // Cache policy of the point streams (used once per stage): 1 marks the
 // stage-output and RK-sum stores evict-first, 2 also the metric, step-start
 // and RK-sum loads, so L2 keeps the plane ring the neighbouring tiles share.
@@ -85,8 +96,9 @@
 // The file is compiled once per tile height -- CG_TILE_Y 4 (an inline
 // namespace, so callers name its functions plainly) and 8 (namespace
 // cgfdm::ty8); a session picks one -- and, the instantiations being many, in
-// several objects: CG_STAGE_SET 0 the ring pipeline, batches and the tensor
-// maps, 1 the split pipeline, 2 mixed storage (4-row tiles only).
+// several objects: CG_STAGE_SET 0 batches and the tensor maps, 1 the split
+// pipeline, 2 mixed storage, 3 halo-linked parts (1 to 3 with 4-row tiles
+// only), 4 the ring pipeline of single sessions.
 #ifndef CG_STAGE_SET
 #define CG_STAGE_SET 0
 #endif
@@ -352,6 +364,19 @@ __device__ __forceinline__ void ljt_z_m(const MixIn &w, const float *__restrict_
     for (int c = 0; c < 3; c++) out[c] = lop(J[0][c], J[1][c], J[2][c], J[3][c], J[4][c], FB, rDH);
 }
 
+// RK4 without the running sum: stage irk's value (irk 0..2) and the step's
+// end from the step start m and the stage values b, c, d.  Every rounding is
+// explicit, so the pipelines agree bit for bit.
+__device__ __forceinline__ float rk_stage(int irk, float m, float h)
+{
+    return irk == 2 ? __fadd_rn(m, h) : __fmaf_rn(RK_ALPHA2, h, m);
+}
+__device__ __forceinline__ float rk_end(float m, float b, float c, float d, float h)
+{
+    const float s = __fadd_rn(__fmaf_rn(2.0f, __fsub_rn(c, m), __fsub_rn(b, m)), __fsub_rn(d, m));
+    return __fadd_rn(m, __fmaf_rn(RK_BETA4, h, __fmul_rn(RK_BETA2, s)));
+}
+
 // a delta to its stored FP16 value (scaled, saturated)
 __device__ __forceinline__ __half to_h16(float x, float sc)
 {
@@ -530,6 +555,12 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                    (long long)kp * g.nx * nPML;
         return (long long)ip + (long long)jp * g.nx + (long long)kp * g.nx * g.ny;
     };
+    // a face's auxiliaries at the stage's input: A, then B B B with a running
+    // sum in T, or B C T (the three stage values) without
+    auto pml_in = [&](const PmlFace &P) -> const float * {
+        if (CG_RK_SUM) return irk == 0 ? P.A : P.B;
+        return irk == 0 ? P.A : irk == 1 ? P.B : irk == 2 ? P.C : P.T;
+    };
     const int item = BATCH ? gitem - item_start[sess] : V2 ? gitem / sweeps : gitem;
     const int sweep = V2 ? gitem - item * sweeps : 0;
     const int tile = item / a.nchunk, chunk = item - tile * a.nchunk;
@@ -596,8 +627,11 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
             if (CG_PREFETCH_MT && irk >= 2) tma_prefetch_4d(tmT, tx0h, ty0, kk, 0);
             return;
         }
-        if (CG_PREFETCH_MT && (irk == 1 || irk == 2)) tma_prefetch_4d(tmM, px0, j0, kk, 0);
-        if (CG_PREFETCH_MT && irk != 0) tma_prefetch_4d(tmT, px0, j0, kk, 0);
+        // the step start; the running sum or, in the last stage, the other two
+        // stage values
+        if (CG_PREFETCH_MT && (irk == 1 || irk == 2 || (irk == 3 && !CG_RK_SUM))) tma_prefetch_4d(tmM, px0, j0, kk, 0);
+        if (CG_PREFETCH_MT && (CG_RK_SUM ? irk != 0 : irk == 3)) tma_prefetch_4d(tmT, px0, j0, kk, 0);
+        if (CG_PREFETCH_MT && !CG_RK_SUM && irk == 3) tma_prefetch_4d(tmS, px0, j0, kk, 0);
     };
     // mixed storage: the delta box of plane kk into its FP32 box, in place,
     // two values at a time (both boxes are [field][row][column], PF values a
@@ -665,7 +699,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
         // point-wise operands, loaded before the ring wait
         float xi_x = 0, et_y = 0, zt_x = 0, zt_y = 0, zt_z = 0;
         float mu = 0, lam = 0, buo = 0, bz = 1;
-        float mv[9], tv[9];
+        float mv[9], tv[9], cv[9];   // step start; running sum, or B and C
         if (active) {
             xi_x = CG_LD(a.cjm[C_XI_X * F + q]), et_y = CG_LD(a.cjm[C_ET_Y * F + q]);
             zt_x = CG_LD(a.cjm[C_ZT_X * F + q]), zt_y = CG_LD(a.cjm[C_ZT_Y * F + q]);
@@ -681,10 +715,12 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                     for (int f = 0; f < 9; f++) tv[f] = __half2float(a.T16[f * a.gh.fstride + qh]) * s_inv[f];
                 }
             } else {
-                if (irk == 1 || irk == 2)
+                if (irk == 1 || irk == 2 || (irk == 3 && !CG_RK_SUM))
                     for (int f = 0; f < 9; f++) mv[f] = CG_LD(a.Wm[f * F + q]);
-                if (irk != 0)
+                if (CG_RK_SUM && irk != 0)
                     for (int f = 0; f < 9; f++) tv[f] = CG_LD(a.T[f * F + q]);
+                if (!CG_RK_SUM && irk == 3)
+                    for (int f = 0; f < 9; f++) tv[f] = CG_LD(a.Wb[f * F + q]), cv[f] = CG_LD(a.Wc[f * F + q]);
             }
         }
         // the first PML face of this point: its operands into the stash
@@ -696,19 +732,26 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                 const PmlFace &P = a.face[fc0];
                 const long long pos = pml_pos(fc0, i, j, k);
                 float *st = stash + ty * TX + tx;
-                const float *cur = irk == 0 ? P.A : P.B;
+                const float *cur = pml_in(P);
+                // the values its RK update reads beside them (see pml_in)
+                const float *o1 = CG_RK_SUM ? (irk != 0 ? P.T : nullptr) : irk == 3 ? P.B : nullptr;
+                const float *o2 = (CG_RK_SUM ? irk == 1 || irk == 2 : irk != 0) ? P.A : nullptr;
                 for (int f = 0; f < 9; f++) cp_async4(st + f * CW, cur + f * P.count + pos);
-                if (NSTASH >= 18 && irk != 0)
-                    for (int f = 0; f < 9; f++) cp_async4(st + (9 + f) * CW, P.T + f * P.count + pos);
-                if (NSTASH >= 27 && (irk == 1 || irk == 2))
-                    for (int f = 0; f < 9; f++) cp_async4(st + (18 + f) * CW, P.A + f * P.count + pos);
+                if (NSTASH >= 18 && o1)
+                    for (int f = 0; f < 9; f++) cp_async4(st + (9 + f) * CW, o1 + f * P.count + pos);
+                if (NSTASH >= 27 && o2)
+                    for (int f = 0; f < 9; f++) cp_async4(st + (18 + f) * CW, o2 + f * P.count + pos);
+                if (NSTASH >= 36 && !CG_RK_SUM && irk == 3)
+                    for (int f = 0; f < 9; f++) cp_async4(st + (27 + f) * CW, P.C + f * P.count + pos);
                 cp_async_commit();
-                // the face's other operands (RK sum, step start) into L2
+                // the face's other operands (RK sum, step start, C) into L2
                 if (CG_PML_REST_PREFETCH) {
-                    if (NSTASH < 18 && irk != 0)
-                        for (int f = 0; f < 9; f++) l2_prefetch(P.T + f * P.count + pos);
-                    if (NSTASH < 27 && (irk == 1 || irk == 2))
-                        for (int f = 0; f < 9; f++) l2_prefetch(P.A + f * P.count + pos);
+                    if (NSTASH < 18 && o1)
+                        for (int f = 0; f < 9; f++) l2_prefetch(o1 + f * P.count + pos);
+                    if (NSTASH < 27 && o2)
+                        for (int f = 0; f < 9; f++) l2_prefetch(o2 + f * P.count + pos);
+                    if (NSTASH < 36 && !CG_RK_SUM && irk == 3)
+                        for (int f = 0; f < 9; f++) l2_prefetch(P.C + f * P.count + pos);
                 }
             }
         }
@@ -875,35 +918,33 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
             if constexpr (DIR == 0) xi_rhs(xi_x, d, mu, lam, buo, rhs);
             else if constexpr (DIR == 1) et_rhs(et_y, d, mu, lam, buo, rhs);
             else dir_rhs(zt_x, zt_y, zt_z, d, mu, lam, buo, rhs);
-            const float *cur = irk == 0 ? P.A : P.B;
+            const float *cur = pml_in(P);
+            constexpr bool SUM = CG_RK_SUM;
+            const bool need_a = SUM ? irk == 1 || irk == 2 : irk != 0;   // the step start
+            const bool need_t = SUM ? irk != 0 : irk == 3;               // the running sum, or B
+            const float *pt = SUM ? P.T : P.B;
             // every operand of this face loaded before the first store: the
             // stores go through pointers the compiler cannot tell apart from
             // the loads, which would otherwise wait for them (8.24 ms per
             // step on 400x400x200 against 8.02 with them first)
-            float xa[9], xt[9];
-            if (STASH && fc == fc0) {
-                cp_async_wait_all();
-                const float *st = stash + ty * TX + tx;
+            float xa[9], xt[9], xc[9];
+            const bool st_ = STASH && fc == fc0;
+            const float *st = stash + ty * TX + tx;
+            if (st_) cp_async_wait_all();
 #pragma unroll
-                for (int f = 0; f < 9; f++) aux[f] = on(f) ? st[f * CW] : 0.0f;
-                if (irk == 1 || irk == 2)
+            for (int f = 0; f < 9; f++) aux[f] = !on(f) ? 0.0f : st_ ? st[f * CW] : cur[f * P.count + pos];
+            if (need_t)
 #pragma unroll
-                    for (int f = 0; f < 9; f++)
-                        xa[f] = !on(f) ? 0.0f : NSTASH >= 27 ? st[(18 + f) * CW] : P.A[f * P.count + pos];
-                if (irk != 0)
+                for (int f = 0; f < 9; f++)
+                    xt[f] = !on(f) ? 0.0f : st_ && NSTASH >= 18 ? st[(9 + f) * CW] : pt[f * P.count + pos];
+            if (need_a)
 #pragma unroll
-                    for (int f = 0; f < 9; f++)
-                        xt[f] = !on(f) ? 0.0f : NSTASH >= 18 ? st[(9 + f) * CW] : P.T[f * P.count + pos];
-            } else {
+                for (int f = 0; f < 9; f++)
+                    xa[f] = !on(f) ? 0.0f : st_ && NSTASH >= 27 ? st[(18 + f) * CW] : P.A[f * P.count + pos];
+            if (!SUM && irk == 3)
 #pragma unroll
-                for (int f = 0; f < 9; f++) aux[f] = on(f) ? cur[f * P.count + pos] : 0.0f;
-                if (irk == 1 || irk == 2)
-#pragma unroll
-                    for (int f = 0; f < 9; f++) xa[f] = on(f) ? P.A[f * P.count + pos] : 0.0f;
-                if (irk != 0)
-#pragma unroll
-                    for (int f = 0; f < 9; f++) xt[f] = on(f) ? P.T[f * P.count + pos] : 0.0f;
-            }
+                for (int f = 0; f < 9; f++)
+                    xc[f] = !on(f) ? 0.0f : st_ && NSTASH >= 36 ? st[(27 + f) * CW] : P.C[f * P.count + pos];
 #pragma unroll
             for (int f = 0; f < 9; f++) hA[f] = (rhs[f] - alpha_d * aux[f]) * DT;
             if (DIR < 2 && surf) {
@@ -920,6 +961,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
 #pragma unroll
             for (int f = 0; f < 9; f++) h[f] = h[f] + (-beta * aux[f]) * DT;
             // src/pml_rk.cpp:18-73
+#if CG_RK_SUM
             if (irk == 0) {
 #pragma unroll
                 for (int f = 0; f < 9; f++)
@@ -939,6 +981,16 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                 for (int f = 0; f < 9; f++)
                     if (on(f)) CG_PST(P.A[f * P.count + pos], xt[f] + RK_BETA4 * hA[f]);
             }
+#else
+            float *out = irk == 0 ? P.B : irk == 1 ? P.C : irk == 2 ? P.T : P.A;
+#pragma unroll
+            for (int f = 0; f < 9; f++) {
+                if (!on(f)) continue;
+                CG_PST(out[f * P.count + pos], irk == 0   ? rk_stage(0, aux[f], hA[f])
+                                               : irk == 3 ? rk_end(xa[f], xt[f], xc[f], aux[f], hA[f])
+                                                          : rk_stage(irk, xa[f], hA[f]));
+            }
+#endif
         };
         unsigned left = (inx1 ? 1u : 0u) | (iny1 ? 2u : 0u) | (inz1 ? 4u : 0u) | (inx2 ? 8u : 0u) | (iny2 ? 16u : 0u);
 #pragma unroll 1
@@ -989,6 +1041,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                 }
             }
         } else {
+#if CG_RK_SUM
         if (irk == 0) {
 #pragma unroll
             for (int f = 0; f < 9; f++) {
@@ -1011,6 +1064,11 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
 #pragma unroll
             for (int f = 0; f < 9; f++) wout[f] = tv[f] + RK_BETA4 * h[f];
         }
+#else
+#pragma unroll
+        for (int f = 0; f < 9; f++)
+            wout[f] = irk == 3 ? rk_end(mv[f], tv[f], cv[f], T.c(f), h[f]) : rk_stage(irk, mv[f], h[f]);
+#endif
 #pragma unroll
         for (int f = 0; f < 9; f++) CG_ST(a.Wout[f * F + q], wout[f]);
         }
@@ -1139,10 +1197,20 @@ cudaError_t launch_cg_stage_split(int FB1, int FB2, int FB3, const CgStageDesc &
 {
     return launch_b<false, false, false, true>(FB1, FB2, FB3, d, nullptr, nullptr, 1, work, ctas, st, d.a.irk);
 }
+#elif CG_STAGE_SET == 3
+cudaError_t launch_cg_stage_part(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int ctas, cudaStream_t st)
+{
+    return launch_b<false, true, false, false>(FB1, FB2, FB3, d, nullptr, nullptr, 1, work, ctas, st, d.a.irk);
+}
+#elif CG_STAGE_SET == 4
+cudaError_t launch_cg_stage(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int ctas, cudaStream_t st)
+{
+    return launch_b<false, false, false, false>(FB1, FB2, FB3, d, nullptr, nullptr, 1, work, ctas, st, d.a.irk);
+}
 #elif CG_STAGE_SET == 2
 cudaError_t launch_cg_stage_mix(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int ctas, cudaStream_t st)
 {
-    return launch_fb<false, false, true, false, -1>(FB1, FB2, FB3, d, nullptr, nullptr, 1, work, ctas, st);
+    return launch_b<false, false, true, false>(FB1, FB2, FB3, d, nullptr, nullptr, 1, work, ctas, st, d.a.irk);
 }
 
 cudaError_t launch_cg_stage_batch_mix(int FB1, int FB2, int FB3, const CgStageDesc *descs, const int *item_start,
@@ -1204,16 +1272,6 @@ cudaError_t launch_impedance_bounds(const float *cjm, DevGrid g, unsigned *out, 
 }
 
 #endif
-
-cudaError_t launch_cg_stage(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int ctas, cudaStream_t st,
-                            bool halo_out)
-{
-#if CG_TILE_Y == 4
-    if (halo_out) return launch_fb<false, true, false, false, -1>(FB1, FB2, FB3, d, nullptr, nullptr, 1, work, ctas, st);
-#endif
-    if (halo_out) return cudaErrorNotSupported;   // parts have 4-row tiles
-    return launch_fb<false, false, false, false, -1>(FB1, FB2, FB3, d, nullptr, nullptr, 1, work, ctas, st);
-}
 
 cudaError_t launch_cg_stage_batch(int FB1, int FB2, int FB3, int irk, const CgStageDesc *descs, const int *item_start,
                                   int nsess, int *work, int ctas, cudaStream_t st)

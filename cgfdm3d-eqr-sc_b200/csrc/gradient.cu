@@ -75,9 +75,8 @@ int Session::load_state(const char *src)
 {
     size_t off = 0, w = sizeof(float) * (size_t)g.fstride * 9;
     CU(cudaMemcpyAsync(W_[0], src, w, cudaMemcpyDeviceToDevice, stream));
-    // the halo of the stage buffers mirrors W_A's (point sources write all three)
-    CU(cudaMemcpyAsync(W_[1], src, w, cudaMemcpyDeviceToDevice, stream));
-    CU(cudaMemcpyAsync(W_[2], src, w, cudaMemcpyDeviceToDevice, stream));
+    // the halo of the stage buffers mirrors W_A's (point sources write all)
+    for (int b = 1; b < (RK_SUM ? 3 : 4); b++) CU(cudaMemcpyAsync(W_[b], src, w, cudaMemcpyDeviceToDevice, stream));
     off += w;
     for (int fc = 0; fc < 5; fc++) {
         size_t b = sizeof(float) * (size_t)face_[fc].count * 9;
@@ -94,7 +93,7 @@ int Session::set_wavefield(const float *host)
     float *d = nullptr;
     CU(cudaMalloc(&d, sizeof(float) * npad * 9));
     cudaError_t e = cudaMemcpyAsync(d, host, sizeof(float) * npad * 9, cudaMemcpyHostToDevice, stream);
-    for (int b = 0; b < 3 && e == cudaSuccess; b++) e = launch_from_aos(d, 9, g, W_[b], stream);
+    for (int b = 0; b < 4 && W_[b] && e == cudaSuccess; b++) e = launch_from_aos(d, 9, g, W_[b], stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     cudaFree(d);
     if (e != cudaSuccess) return cuda_fail(e, "set_wavefield");
@@ -146,6 +145,7 @@ int Session::set_medium(const float *host)
             CU(cudaMemsetAsync(face_[fc].A, 0, b, stream));
             CU(cudaMemsetAsync(face_[fc].B, 0, b, stream));
             CU(cudaMemsetAsync(face_[fc].T, 0, b, stream));
+            if (face_[fc].C) CU(cudaMemsetAsync(face_[fc].C, 0, b, stream));
         }
     CU(cudaMemsetAsync(pgv_, 0, sizeof(float) * m.g.nx * m.g.ny * 2, stream));
     if (pga_) CU(cudaMemsetAsync(pga_, 0, sizeof(float) * m.g.nx * m.g.ny * 2, stream));

@@ -87,10 +87,10 @@ int Session::halo_copy(int face, int which, float *dev, bool pack)
     return ST_OK;
 }
 
-int Session::link_halo_to(int face, float *const nw[3], const DevGrid &ng)
+int Session::link_halo_to(int face, float *const nw[4], const DevGrid &ng)
 {
     if (int st = need_fp32_storage("link_halo_to")) return st;
-    if (face < 0 || face > 5 || m.p.scheme != SCHEME_CGFDM || !nw[0] || !nw[1] || !nw[2]) {
+    if (face < 0 || face > 5 || m.p.scheme != SCHEME_CGFDM || !nw[0] || !nw[1] || !nw[2] || !nw[3]) {
         err = "bad face, scheme or buffers for a halo link";
         return ST_ARG;
     }
@@ -104,10 +104,9 @@ int Session::link_halo_to(int face, float *const nw[3], const DevGrid &ng)
         err = "the neighbour's grid does not match on the shared face";
         return ST_ARG;
     }
-    static const int wout[4] = {1, 2, 1, 0};   // output buffer of RK stage irk
     for (int irk = 0; irk < 4; irk++) {
         HaloOut &h = ho_[irk][face];
-        h.base = nw[wout[irk]];
+        h.base = nw[STAGE_OUT[irk]];
         h.plane = ng.plane, h.fstride = ng.fstride;
         h.pitch = ng.pitch, h.xoff = ng.xoff;
         // high face: interior n_self..n_self+2 -> neighbour halo 0..2;
@@ -124,14 +123,14 @@ int Session::link_halo(int face, const Session &nbr)
         err = "the neighbour is not a CGFDM part";
         return ST_ARG;
     }
-    float *const nw[3] = {nbr.W_[0], nbr.W_[1], nbr.W_[2]};
+    float *const nw[4] = {nbr.W_[0], nbr.W_[1], nbr.W_[2], nbr.W_[3]};
     return link_halo_to(face, nw, nbr.g);
 }
 
 // A part's stage buffers for a neighbour in another process: CUDA IPC
-// handles of buffers A, B, C and their layout.
+// handles of buffers A, B, C, D and their layout.
 struct PartHandle {
-    cudaIpcMemHandle_t w[3];
+    cudaIpcMemHandle_t w[4];
     DevGrid g;
     long long magic;
 };
@@ -147,7 +146,7 @@ int Session::part_handle(void *out, long long bytes)
     }
     PartHandle h;
     std::memset(&h, 0, sizeof h);
-    for (int b = 0; b < 3; b++) CU(cudaIpcGetMemHandle(&h.w[b], W_[b]));
+    for (int b = 0; b < 4; b++) CU(cudaIpcGetMemHandle(&h.w[b], W_[b]));
     h.g = g;
     h.magic = PART_HANDLE_MAGIC;
     std::memcpy(out, &h, sizeof h);
@@ -167,8 +166,8 @@ int Session::link_halo_handle(int face, const void *handle, long long bytes)
         return ST_ARG;
     }
     CU(cudaSetDevice(device));
-    float *nw[3];
-    for (int b = 0; b < 3; b++) {
+    float *nw[4];
+    for (int b = 0; b < 4; b++) {
         void *p = nullptr;
         CU(cudaIpcOpenMemHandle(&p, h.w[b], cudaIpcMemLazyEnablePeerAccess));
         ipc_open_.push_back(p);
@@ -202,7 +201,7 @@ int Session::create_part(const std::string &dir, const std::string &options, con
 }
 
 // One phase of a part's step: 0 the source of step `it` into the step-start
-// state A, 1..4 RK stage 0..3 (A -> B -> C -> B -> A); after stage 3 the
+// state A, 1..4 RK stage 0..3 (STAGE_OUT); after stage 3 the
 // stations record and the step is done.  cur_ names the buffer the phase
 // wrote, the one the halo exchange refreshes.
 int Session::part_advance(int *phase_done)
@@ -243,11 +242,10 @@ int Session::part_launch(int *phase_done)
         int fb[3];
         fb_signs(it, fb);
         const int sgn = (irk & 1) ? -1 : 1;
-        CU(launch_cg_stage(fb[0] * sgn, fb[1] * sgn, fb[2] * sgn, desc_host_[irk], work_dev_, grid_ctas_, stream,
-                           halo_out_));
+        auto launch = halo_out_ ? launch_cg_stage_part : launch_cg_stage;
+        CU(launch(fb[0] * sgn, fb[1] * sgn, fb[2] * sgn, desc_host_[irk], work_dev_, grid_ctas_, stream));
         kernel_launches += 1;
-        static const int wout[4] = {1, 2, 1, 0};
-        cur_ = wout[irk];
+        cur_ = STAGE_OUT[irk];
         if (irk == 3) {
             if (int st = launch_pga_on(stream)) return st;
             if (int st = launch_stations_on(stream)) return st;

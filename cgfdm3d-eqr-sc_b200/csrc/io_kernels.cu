@@ -64,9 +64,9 @@ __global__ void k_fault(float *W, const float *__restrict__ cjm, DevGrid g, Faul
 
 // Single point source, 7x7x7 Gaussian-smoothed (src/singleSource.cpp:111-173
 // Ricker, explosive; :216-318 double couple).  Cells inside the halo also
-// receive the value in the stage buffers (B, C), because the reference's RK
+// receive the value in the stage buffers (B, C, D), because the reference's RK
 // update keeps halo cells at their step-start value through all stages.
-__global__ void k_point(float *W, float *Wb, float *Wc, const float *__restrict__ cjm, DevGrid g, PointDev p,
+__global__ void k_point(float *W, float *Wb, float *Wc, float *Wd, const float *__restrict__ cjm, DevGrid g, PointDev p,
                         const int *it_dev, float DT, float DH, int scheme, float *Walt, unsigned *mx)
 {
     const int t = threadIdx.x;
@@ -77,7 +77,7 @@ __global__ void k_point(float *W, float *Wb, float *Wc, const float *__restrict_
         // cells, which no stage updates, get the value in both
         Wb = (it & 1) ? W : Walt;
         W = (it & 1) ? Walt : W;
-        Wc = nullptr;
+        Wc = Wd = nullptr;
     }
     const int di = t % 7 - 3, dj = (t / 7) % 7 - 3, dk = t / 49 - 3;
     const int i = p.X + di, j = p.Y + dj, k = p.Z + dk;
@@ -130,6 +130,7 @@ __global__ void k_point(float *W, float *Wb, float *Wc, const float *__restrict_
         if (halo) {
             if (Wb) Wb[(3 + c) * F + q] = v;
             if (Wc) Wc[(3 + c) * F + q] = v;
+            if (Wd) Wd[(3 + c) * F + q] = v;
         } else if (mx) {
             atomicMax(&mx[(it & 1) * 9 + 3 + c], __float_as_uint(fabsf(v)));
         }
@@ -148,11 +149,11 @@ cudaError_t launch_sources(float *W, const float *cjm, DevGrid g, const FaultDev
     return cudaSuccess;
 }
 
-cudaError_t launch_point(float *W, float *Wb, float *Wc, const float *cjm, DevGrid g, const PointDev &p,
+cudaError_t launch_point(float *W, float *Wb, float *Wc, float *Wd, const float *cjm, DevGrid g, const PointDev &p,
                          const int *it_dev, float DT, float DH, int scheme, cudaStream_t st, float *Walt, unsigned *mx)
 {
     if (p.kind == 0 || !p.inside) return cudaSuccess;
-    k_point<<<1, 352, 0, st>>>(W, Wb, Wc, cjm, g, p, it_dev, DT, DH, scheme, Walt, mx);
+    k_point<<<1, 352, 0, st>>>(W, Wb, Wc, Wd, cjm, g, p, it_dev, DT, DH, scheme, Walt, mx);
     return cudaGetLastError();
 }
 

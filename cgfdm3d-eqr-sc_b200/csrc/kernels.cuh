@@ -19,11 +19,12 @@ cudaError_t launch_scale_moment(float *rate, const long long *cell, long long np
                                 DevGrid g, float DH, cudaStream_t st);
 
 // ------------------------------------------------------------ PML state
-// One absorbing face: Aux fields for its slab, three buffers (A holds the
-// step-start value and receives the final stage, B the intermediate stage
-// values, T the RK accumulator), each 9 fields of `count` floats.
+// One absorbing face: Aux fields for its slab, each buffer 9 fields of
+// `count` floats.  A holds the step-start value and receives the final stage;
+// B, C and T the values of stages 0, 1 and 2 or, in the exact build, B every
+// stage's and T the RK accumulator (no C).
 struct PmlFace {
-    float *A, *B, *T;
+    float *A, *B, *T, *C;
     long long count;     // points in the slab
     int n0, n1;          // slab extent along its two fastest axes (see pml_pos)
 };
@@ -60,7 +61,8 @@ struct CgStageArgs {
     HBox hbox;           // layout of hstore
     const float *Win;    // stencil input of this stage
     const float *Wm;     // values at the start of the step (RK "m")
-    float *T;            // RK accumulator
+    float *T;            // RK accumulator (exact build)
+    const float *Wb, *Wc;  // the values of stages 0 and 1, for the last stage (default build)
     float *Wout;         // stage output
     const float *cjm;    // 13 fields
     const float *rdz;    // 18 surface fields [nyp][pitch]
@@ -116,14 +118,14 @@ struct CgStageMaps {
     alignas(64) unsigned char win[128];
     alignas(64) unsigned char cjm[128], cjm1[128];   // metric and medium: boxes of 3 fields and of 1 field
     alignas(64) unsigned char wm[128];
-    alignas(64) unsigned char t[128];
+    alignas(64) unsigned char t[128], c[128];   // T or B, and C
 };
 // Everything one stage launch needs for one session: the tensor maps
 // (CUtensorMap, 128 bytes each, 64-byte aligned) and the arguments.
 // work: the launch's work-counter pair, zero between launches.
 struct alignas(64) CgStageDesc {
     unsigned char tmW[128], tmC[128], tmC1[128], tmM[128], tmT[128];
-    unsigned char tmS[128];   // mixed storage: the FP16 stencil-input delta, halo box
+    unsigned char tmS[128];   // mixed storage: the FP16 stencil-input delta, halo box; else C's point box
     unsigned char tmWc[128];  // split pipeline: the stencil input, interior column box
     CgStageArgs a;
 };
@@ -138,6 +140,7 @@ struct alignas(64) CgStageDesc {
 // launch_cg_stage_split: the split pipeline (the current plane's halo box,
 // interior column boxes for the z window): one session's FP32 stage, a.sweeps
 // 4-row sweeps an item (namespace ty4 only).
+// launch_cg_stage_part: the ring pipeline storing into linked parts' halos.
 // launch_cg_stage_mix: mixed-precision storage (the MIX instantiation);
 // launch_cg_stage_batch_mix: the same for a batch of such sessions.
 // make_field_tmap16: FP16 counterpart of make_field_tmap (halo box), for
@@ -150,7 +153,9 @@ struct alignas(64) CgStageDesc {
 // when given; out must hold 128 bytes.
 #define CG_STAGE_FUNCTIONS                                                                                         \
     cudaError_t launch_cg_stage(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,      \
-                                cudaStream_t st, bool halo_out = false);                                         \
+                                cudaStream_t st);                                                                \
+    cudaError_t launch_cg_stage_part(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas, \
+                                     cudaStream_t st);                                                           \
     cudaError_t launch_cg_stage_batch(int FB1, int FB2, int FB3, int irk, const CgStageDesc *descs,               \
                                       const int *item_start, int nsess, int *work, int grid_ctas,                 \
                                       cudaStream_t st);                                                          \
@@ -288,7 +293,7 @@ struct PointDev {
 cudaError_t launch_sources(float *W, const float *cjm, DevGrid g, const FaultDev &f, const PointDev &p,
                            const int *it_dev, float DT, float DH, int scheme, cudaStream_t st,
                            float *Walt = nullptr, unsigned *mx = nullptr);
-cudaError_t launch_point(float *W, float *Wb, float *Wc, const float *cjm, DevGrid g, const PointDev &p,
+cudaError_t launch_point(float *W, float *Wb, float *Wc, float *Wd, const float *cjm, DevGrid g, const PointDev &p,
                          const int *it_dev, float DT, float DH, int scheme, cudaStream_t st, float *Walt = nullptr,
                          unsigned *mx = nullptr);
 // Records 9 components per station at step *it_dev, then advances *it_dev.

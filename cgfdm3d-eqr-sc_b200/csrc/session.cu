@@ -237,7 +237,7 @@ size_t Session::arena_estimate() const
                                    nP * G.nx * G.nz};
             for (int fc = 0; fc < 5; fc++)
                 if (pml_faces() & (1 << fc))
-                    for (int x = 0; x < 3; x++) add(sizeof(float) * cnt[fc] * 9);
+                    for (int x = 0; x < (RK_SUM ? 3 : 4); x++) add(sizeof(float) * cnt[fc] * 9);
         }
     }
     add(sizeof(float) * (size_t)G.nx * G.ny * 2);
@@ -426,6 +426,7 @@ int Session::setup_device()
             ALLOC(face_[fc].A, float, cnt[fc] * 9);
             ALLOC(face_[fc].B, float, cnt[fc] * 9);
             ALLOC(face_[fc].T, float, cnt[fc] * 9);
+            if (!RK_SUM) ALLOC(face_[fc].C, float, cnt[fc] * 9);
         }
     } else if (cg) {
         // PML off: unit stretching, zero damping
@@ -546,21 +547,19 @@ int stage_chunk(long long tiles, int nz, int ctas)
     return (nz + n - 1) / n;
 }
 
-// The four stage descriptors (RK4 stage irk reads win[irk] and writes
-// wout[irk]: A -> B, B -> C, C -> B, B -> A) with their tensor maps.
+// The four stage descriptors (RK4 stage irk reads buffer STAGE_IN[irk] and
+// writes STAGE_OUT[irk]) with their tensor maps.
 void Session::stage_desc(int irk, CgStageDesc &d, bool batched) const
 {
-    float *A = W_[0], *B = W_[1], *C = W_[2], *T = W_[3];
-    const float *win[4] = {A, B, C, B};
-    const int win_map[4] = {0, 1, 2, 1};
-    float *wout[4] = {B, C, B, A};
+    float *A = W_[0], *T = W_[3];
     std::memset(&d, 0, sizeof d);
     CgStageArgs &a = d.a;
     a.g = g;
-    a.Win = win[irk];
+    a.Win = W_[STAGE_IN[irk]];
     a.Wm = A;
     a.T = T;
-    a.Wout = wout[irk];
+    a.Wout = W_[STAGE_OUT[irk]];
+    a.Wb = W_[1], a.Wc = W_[2];
     a.cjm = cjm_;
     a.rdz = rdz_;
     a.pml_alpha_x = pml_[0], a.pml_beta_x = pml_[1], a.pml_d_x = pml_[2];
@@ -584,13 +583,14 @@ void Session::stage_desc(int irk, CgStageDesc &d, bool batched) const
     a.ntiles_x = ntx_, a.ntiles_y = nty_, a.nchunk = nchunk_;
     a.sweeps = tile_ / 4;
     for (int f = 0; f < 6; f++) a.ho[f] = ho_[irk][f];
-    const CgStageMaps &M = (split() && !batched ? split_maps_ : maps_)[win_map[irk]];
+    const CgStageMaps &M = (split() && !batched ? split_maps_ : maps_)[STAGE_IN[irk]];
     std::memcpy(d.tmW, M.win, 128);
     std::memcpy(d.tmC, M.cjm, 128);
     std::memcpy(d.tmC1, M.cjm1, 128);
     std::memcpy(d.tmM, M.wm, 128);
     std::memcpy(d.tmT, M.t, 128);
     std::memcpy(d.tmWc, M.winp, 128);
+    std::memcpy(d.tmS, M.c, 128);
 }
 
 // (the split pipeline hands an item's 4-row sweeps out one by one)
@@ -622,14 +622,15 @@ int Session::build_maps()
             return eight ? ty8::make_field_tmap(out, base, g, nf, halo, box_nf)
                          : make_field_tmap(out, base, g, nf, halo, box_nf);
         };
-        for (int b = 0; b < 3; b++) {
+        for (int b = 0; b < 4; b++) {
             CgStageMaps &M = (split_set ? split_maps_ : maps_)[b];
             CU(tmap(M.win, W_[b], 9, true));
             CU(tmap(M.winp, W_[b], 9, false));
             CU(tmap(M.cjm, cjm_, 13, false, 3));
             CU(tmap(M.cjm1, cjm_, 13, false, 1));
             CU(tmap(M.wm, W_[0], 9, false));
-            CU(tmap(M.t, W_[3], 9, false));
+            CU(tmap(M.t, RK_SUM ? W_[3] : W_[1], 9, false));
+            CU(tmap(M.c, W_[2], 9, false));
         }
     }
     return ST_OK;
@@ -788,11 +789,11 @@ int Session::launch_sources_on(cudaStream_t st)
 {
     const float DT = (float)m.p.DT;
     if (mix_) {
-        CU(launch_point(W_[0], nullptr, nullptr, cjm_, g, point_, it_dev_, DT, m.g.DH, m.p.scheme, st, Walt_, mx_));
+        CU(launch_point(W_[0], nullptr, nullptr, nullptr, cjm_, g, point_, it_dev_, DT, m.g.DH, m.p.scheme, st, Walt_, mx_));
         CU(launch_sources(W_[0], cjm_, g, fault_, point_, it_dev_, DT, m.g.DH, m.p.scheme, st, Walt_, mx_));
         return ST_OK;
     }
-    CU(launch_point(W_[0], W_[1], W_[2], cjm_, g, point_, it_dev_, DT, m.g.DH, m.p.scheme, st));
+    CU(launch_point(W_[0], W_[1], W_[2], W_[3], cjm_, g, point_, it_dev_, DT, m.g.DH, m.p.scheme, st));
     CU(launch_sources(W_[0], cjm_, g, fault_, point_, it_dev_, DT, m.g.DH, m.p.scheme, st));
     return ST_OK;
 }
@@ -971,11 +972,9 @@ int Session::profile_stages(int nsteps, float *mean)
     return check_device_error();
 }
 
-// Minimum bytes a step moves (float fields of 4 bytes): RK4 stages read the
-// stencil input, 12 metric/medium fields and the RK state and write the stage
-// output and accumulator, 39 + 57 + 57 + 39 = 192 fields per interior point;
-// each absorbing face adds 27 + 45 + 45 + 27 = 144 auxiliary fields per slab
-// point.
+// Minimum bytes a step moves (float fields of 4 bytes): every stage reads its
+// stencil input, eight metric and medium fields and the RK operands and
+// writes its value (and the running sum where there is one).
 double Session::algo_bytes_per_step() const
 {
     const Grid &G = m.g;
@@ -984,18 +983,18 @@ double Session::algo_bytes_per_step() const
     // SCFDM: W_n + 13 metric/medium fields -> W1 (31 fields), then two stages
     // reading the stage value, the metric and W_n and writing W (40 each)
     if (m.p.scheme == SCHEME_SCFDM) return 4.0 * 111.0 * n;
-    // FP16 storage: 4-byte state and metric fields, 2-byte deltas; stage 0
-    // reads A and 12 metric fields and writes the delta (84 + 18 B), stage 1
-    // adds the delta in and writes the accumulator and the next delta (102 +
-    // 36), stages 2-3 also read the accumulator (120 + 36); stage 3 writes
-    // the 4-byte state (120 + 36): 552 B per point and step
-    if (mix_) {
-        if (m.p.pml) faces = (double)G.nPML * (2.0 * G.ny * G.nz + 2.0 * G.nx * G.nz + (double)G.nx * G.ny);
-        return 552.0 * n + 4.0 * 144.0 * faces;
-    }
-    if (m.p.pml && m.p.scheme == SCHEME_CGFDM)
-        faces = (double)G.nPML * (2.0 * G.ny * G.nz + 2.0 * G.nx * G.nz + (double)G.nx * G.ny);
-    return 4.0 * (192.0 * n + 144.0 * faces);
+    if (m.p.pml) faces = (double)G.nPML * (2.0 * G.ny * G.nz + 2.0 * G.nx * G.nz + (double)G.nx * G.ny);
+    // an absorbing-layer point's auxiliaries: 27 + 45 + 45 + 27 fields with a
+    // running sum, 18 + 27 + 27 + 45 without
+    const double aux = 4.0 * (RK_SUM ? 144.0 : 117.0) * faces;
+    // FP16 storage: 4-byte state and eight metric fields, 2-byte deltas; stage
+    // 0 reads A and the metric and writes the delta (68 + 18 B), stage 1 adds
+    // the delta in and writes the accumulator and the next delta (86 + 36),
+    // stages 2-3 also read the accumulator (104 + 36); stage 3 writes the
+    // 4-byte state (104 + 36): 488 B per point and step
+    if (mix_) return 488.0 * n + aux;
+    // 26 + 35 + 35 + 53 fields, or 35 + 53 + 53 + 35 with a running sum
+    return 4.0 * (RK_SUM ? 176.0 : 149.0) * n + aux;
 }
 
 // ------------------------------------------------------------- readback

@@ -20,6 +20,17 @@ void fb_signs(int step, int fb[3]);
 void arena_session_add(int device);
 void arena_session_remove(int device);
 
+// CGFDM wavefield buffers A, B, C, D by RK stage: A -> B, B -> C, C -> D, D ->
+// A, the last stage combining all four.  The exact build keeps the reference's
+// running sum in the fourth buffer instead: A -> B, B -> C, C -> B, B -> A.
+#ifdef CGFDM_EXACT
+constexpr bool RK_SUM = true;
+constexpr int STAGE_IN[4] = {0, 1, 2, 1}, STAGE_OUT[4] = {1, 2, 1, 0};
+#else
+constexpr bool RK_SUM = false;
+constexpr int STAGE_IN[4] = {0, 1, 2, 3}, STAGE_OUT[4] = {1, 2, 3, 0};
+#endif
+
 // planes per work item of a stage launch (csrc/session.cu)
 int stage_chunk(long long tiles, int nz, int ctas);
 
@@ -49,7 +60,7 @@ public:
     // part's halo directly (same device, or peer memory): the halo exchange
     // of phases 1..4 folded into the stages
     int link_halo(int face, const Session &nbr);
-    int link_halo_to(int face, float *const nbr_w[3], const DevGrid &nbr_g);
+    int link_halo_to(int face, float *const nbr_w[4], const DevGrid &nbr_g);
     // the same across processes: CUDA IPC handles of the stage buffers
     int part_handle(void *out, long long bytes);
     int link_halo_handle(int face, const void *handle, long long bytes);
@@ -141,7 +152,7 @@ private:
     char *arena_ = nullptr;
     size_t arena_size_ = 0, arena_used_ = 0;
     size_t arena_estimate() const;
-    float *W_[4] = {nullptr, nullptr, nullptr, nullptr};  // A B C T
+    float *W_[4] = {nullptr, nullptr, nullptr, nullptr};  // A B C D (exact build: A B C T)
     float *cjm_ = nullptr, *rdz_ = nullptr;
     float *pml_[9] = {};
     PmlFace face_[5] = {};
@@ -156,7 +167,7 @@ private:
     cudaGraphExec_t graph8_ = nullptr;
     cudaGraph_t graph8_src_ = nullptr;
     cudaEvent_t ev_[4] = {};
-    CgStageMaps maps_[3] = {}, split_maps_[3] = {};  // TMA descriptors per stencil input A, B, C
+    CgStageMaps maps_[4] = {}, split_maps_[4] = {};  // TMA descriptors per stencil input A, B, C, D
     CgStageDesc desc_host_[4] = {};                  // stage descriptors, one per RK stage
     int build_stage_descs();
     int *work_dev_ = nullptr;                        // persistent-CTA work counters

@@ -169,9 +169,10 @@ int cgfdm_info_get(const cgfdm_session *s, cgfdm_info *out);
  * CUDA events around each fused stage kernel, and returns the mean device
  * time of one stage launch in milliseconds.  Divide algo_bytes_per_step by
  * stage_kernels_per_step for the algorithmic bytes of one launch: per
- * interior point and step, the stencil input, metric and medium (12 fields),
- * RK state and accumulator of every stage (192 float fields in all for
- * RK4), plus 144 auxiliary fields per point of each absorbing face. */
+ * interior point and step, the stencil input, metric and medium (8 fields that
+ * are not zero on vertical columns) and the RK operands of every stage (149
+ * float fields in all for RK4, 176 in the exact build, which keeps a running
+ * sum), plus 117 (144) auxiliary fields per point of each absorbing face. */
 int cgfdm_profile_stages(cgfdm_session *s, int nsteps, float *mean_stage_ms);
 
 /* Station traces, [n_stations][NT][9] as the reference stores them
