@@ -21,16 +21,21 @@ import torch
 from . import Session
 
 
-def _padded_medium(vp: np.ndarray, vs: np.ndarray, rho: np.ndarray) -> np.ndarray:
-    med = np.stack([vs, vp, rho], axis=-1).astype(np.float32)
-    return np.pad(med, ((3, 3), (3, 3), (3, 3), (0, 0)), mode="edge")
+def _padded_medium(vp: torch.Tensor, vs: torch.Tensor, rho: torch.Tensor) -> np.ndarray:
+    """(Vs, Vp, rho) [nzp][nyp][nxp][3] on the host, the halo filled from the
+    nearest interior point.  Stacked and padded on vp's device, so that one
+    copy brings the finished volume."""
+    if not vp.shape == vs.shape == rho.shape or vp.dim() != 3:
+        raise ValueError("vp, vs and rho must have one shape [nz][ny][nx]")
+    m = torch.stack([t.detach().to(vp.device, torch.float32) for t in (vs, vp, rho)])
+    m = torch.nn.functional.pad(m[None], (3,) * 6, mode="replicate")[0]
+    return m.permute(1, 2, 3, 0).contiguous().cpu().numpy()
 
 
 class SeismogramMisfit(torch.autograd.Function):
     @staticmethod
     def forward(ctx, vp, vs, rho, session: Session, observed, checkpoint_every: int = 100):
-        host = [t.detach().to("cpu", torch.float32).numpy() for t in (vp, vs, rho)]
-        session.set_medium(_padded_medium(*host))
+        session.set_medium(_padded_medium(vp, vs, rho))
         obs = observed.detach().to("cpu", torch.float32).numpy() if torch.is_tensor(observed) else observed
         if any(ctx.needs_input_grad[:3]):
             J, g = session.gradient(obs, checkpoint_every)

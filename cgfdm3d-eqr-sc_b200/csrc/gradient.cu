@@ -108,23 +108,31 @@ int Session::set_medium(const float *host)
         return ST_OPTIONS;
     }
     const long long npad = m.g.npad();
-    FieldVec old = m.medium;
-    m.medium.assign(host, host + npad * 3);
-    float vpmax = 0.0f;
-    for (long long n = 0; n < npad; n++) vpmax = std::max(vpmax, m.medium[n * 3 + 1]);
+    const float vpmax = medium_vp_max(host, m.g);
     if ((float)m.p.DT > (float)(1.34 * m.H_min / vpmax)) {
-        m.medium.swap(old);
         err = "the new medium violates the CFL condition at this DT";
         return ST_CFL;
     }
+    copy_medium(m, host);
     m.Vp_max = vpmax;
     m.dtmax = (float)(1.34 * m.H_min / m.Vp_max);
-    materialize_coords(m);   // the set-up kernels take the coordinate volume
-    float *d_coord = nullptr, *d_med = nullptr;
+    // the coordinates the set-up kernels take are made from the height map, as
+    // at creation (a part's sub-block of the volume is uploaded)
+    const Grid &G = m.g;
+    float *d_coord = nullptr, *d_med = nullptr, *d_terrain = nullptr;
     CU(cudaMalloc(&d_coord, sizeof(float) * npad * 3));
     cudaError_t e = cudaMalloc(&d_med, sizeof(float) * npad * 3);
-    if (e == cudaSuccess)
+    if (m.coord_mode >= 0) {
+        const size_t tb = sizeof(float) * (size_t)G._nx_ * G._ny_;
+        if (e == cudaSuccess) e = cudaMalloc(&d_terrain, tb);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d_terrain, m.terrain.data(), tb, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess)
+            e = launch_build_coords(d_coord, d_terrain, G._nx_, G._ny_, G._nz_, m.coord_mode, G.DH, G.originalX,
+                                    G.originalY, G.NZ, m.coord_depth_f, m.coord_depth_d, stream);
+    } else if (e == cudaSuccess) {
+        materialize_coords(m);
         e = cudaMemcpyAsync(d_coord, m.coord.data(), sizeof(float) * npad * 3, cudaMemcpyHostToDevice, stream);
+    }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_med, m.medium.data(), sizeof(float) * npad * 3, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = launch_setup(d_coord, d_med, cjm_, rdz_, g, m.g.rDH, m.p.scheme, m.p.metric_fp64, stream);
@@ -136,6 +144,7 @@ int Session::set_medium(const float *host)
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     cudaFree(d_coord);
     cudaFree(d_med);
+    cudaFree(d_terrain);
     if (e != cudaSuccess) return cuda_fail(e, "set_medium");
     // back to step 0
     for (int b = 0; b < 4; b++) CU(cudaMemsetAsync(W_[b], 0, sizeof(float) * g.fstride * 9, stream));

@@ -866,6 +866,27 @@ static int medium_file(Model &m, const std::string &path, std::string &err)
     return ST_OK;
 }
 
+float medium_vp_max(const float *medium, const Grid &g)
+{
+    const long long plane = (long long)g._nx_ * g._ny_;
+    std::vector<float> mx((size_t)g._nz_, 0.0f);
+    par_for(g._nz_, [&](int k) {
+        float v = 0.0f;
+        for (long long q = k * plane; q < (k + 1) * plane; q++) v = std::max(v, medium[q * 3 + 1]);
+        mx[(size_t)k] = v;
+    });
+    float v = 0.0f;
+    for (float x : mx) v = std::max(v, x);
+    return v;
+}
+
+void copy_medium(Model &m, const float *medium)
+{
+    const size_t plane = (size_t)m.g._nx_ * m.g._ny_ * 3;
+    m.medium.resize(plane * m.g._nz_);   // every value written below
+    par_for(m.g._nz_, [&](int k) { std::memcpy(m.medium.data() + k * plane, medium + k * plane, plane * sizeof(float)); });
+}
+
 static void value_ranges(Model &m)
 {
     // src/calc_CFL.cpp:165-180,283-285: ranges over the whole padded grid

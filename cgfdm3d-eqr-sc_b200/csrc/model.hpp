@@ -239,6 +239,10 @@ void point_moment(float strike, float dip, float rake, float Mw, float mom[6], f
 // faces at the global boundary only, the free surface in the top layer of
 // parts, sources and stations of the part's interior.  CGFDM only.
 int slice_model(const Model &G, const int parts[3], const int coord[3], Model &m, std::string &err);
+// the largest Vp of a medium volume [_nz_][_ny_][_nx_][3] (0 at least), and
+// the model's own copy of one, both plane by plane on the host's cores
+float medium_vp_max(const float *medium, const Grid &g);
+void copy_medium(Model &m, const float *medium);
 // fills m.coord if it was left to coord_at (no-op otherwise)
 void materialize_coords(Model &m);
 // interior offset and size of part c of n along an axis of N points
