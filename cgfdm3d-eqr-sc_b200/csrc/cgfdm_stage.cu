@@ -13,22 +13,31 @@
 // velocity (src/PGV.cpp:61-175) and, if enabled, the displacement
 // (src/solve_displacement.cpp:27-63).
 //
-// Tiling: a CTA owns a 32 x 4 column tile and marches up a chunk of z.  Each
-// z-plane of the nine stencil-input components, with the halo the one-sided
-// operators need, arrives as one TMA box (40 x 8 x 1 x 9 floats,
-// cp.async.bulk.tensor.4d) into a six-slot shared-memory ring, completion
-// tracked by one mbarrier per slot; one elected thread issues the copies one
-// plane ahead of use.  Derivatives along x, y and z all read the ring, so
-// each value crosses HBM once per stage.  The FB signs are template
-// parameters, so every stencil tap is a fixed shared-memory offset.  Metric,
-// medium and RK inputs are plain coalesced loads issued before the ring wait.
+// Tiling: a CTA owns a 32 x 4 column tile and marches up a chunk of z.  Only
+// the current plane needs its x/y halo: it arrives as one TMA box (40 x 8 x 1 x
+// 9 floats, cp.async.bulk.tensor.4d) in a two-slot ring, and every plane of
+// the one-sided z window as an interior column box (32 x 4 x 1 x 9) in a
+// six-slot ring, completion tracked by one mbarrier per slot; one elected
+// thread issues the copies one plane ahead of use.  (The ring pipeline of
+// batches and linked parts brings every plane as a halo box in one six-slot
+// ring.)  The FB signs are template parameters, so every stencil tap is a
+// fixed shared-memory offset.  Metric, medium and RK inputs are plain
+// coalesced loads issued before the ring wait.
+//
+// What bounds it: 400 x 400 x 200, the default build, moves 24 GB a step in
+// 6.35 ms (3.8 TB/s of algorithmic bytes; DRAM at 60 % of its nominal peak in
+// the middle stages, issue slots 45-50 % full, the rest waits for memory with
+// twelve warps an SM).  Before the zero metric terms, the factored sums and
+// the running sum's going it was 8.2 ms, 1174-1304 instructions a warp of
+// points against 830-960 now.
 //
 // Every wait on an mbarrier is bounded: on timeout the CTA records the fact
 // in a device error word, waits (bounded) for its copies in flight and exits.
 //
-// Arithmetic follows the reference's expression order term by term; built
-// with --fmad=false the stage reproduces the reference's FP32 results bit for
-// bit, built normally it differs only by FMA contraction.
+// The exact build (CGFDM_EXACT, --fmad=false) follows the reference's
+// expression order term by term and reproduces its FP32 results bit for bit;
+// the default build factors the sums and ends the RK step without a running
+// sum, and is no further from FP64.
 #include <type_traits>
 
 #include "cg_ops.cuh"
@@ -112,11 +121,10 @@
 namespace cgfdm {
 CG_TILE_NS_INLINE namespace CG_TILE_NS {
 
-// 32 x 4 tiles, three CTAs per SM (12 warps, 168 registers): 5 % faster on
-// the 400 x 400 x 200 workload than 32 x 8 tiles at two CTAs per SM, the
-// three independent per-plane barriers hiding more load latency.  A variant
-// that also brought the point operands in by TMA (a second ring) lost
-// occupancy and was 9 % slower.
+// 32 x 4 tiles, three CTAs per SM (12 warps, 168 registers): on 400 x 400 x
+// 200 6.95 ms per step against 7.43 for 32 x 8 tiles at two CTAs of 128
+// registers, which spill, and 7.07 for 128 threads of two points each in
+// packed arithmetic (8 warps).
 #ifndef CG_TILE_Y
 #define CG_TILE_Y 4      // rows per tile (threads per CTA = 32 x CG_TILE_Y)
 #endif
@@ -135,9 +143,8 @@ CG_TILE_NS_INLINE namespace CG_TILE_NS {
 #define SLOT_BYTES (SLOT_F * 4)
 #define NSLOT 6
 // split pipeline: the current plane's halo box in a 2-slot ring, the
-// z-window's interior column boxes (32 x TY x 9) in a 6-slot ring, and the
-// point operands (13 metric/medium + 9 step-start + 9 RK-sum fields) of the
-// current plane in one slot
+// z-window's interior column boxes (32 x TY x 9) in a 6-slot ring (three and
+// seven slots, a plane more ahead: 5 % slower)
 #define CW (TX * TY)
 #define CSLOT_F (9 * CW)
 #define CSLOT_BYTES (CSLOT_F * 4)
@@ -149,31 +156,6 @@ CG_TILE_NS_INLINE namespace CG_TILE_NS {
 #endif
 #define NHSLOT CG_SPLIT_HSLOTS
 #define NCSLOT CG_SPLIT_CSLOTS
-// Split pipeline: the first PML face of each PML point has its operands
-// copied into a per-thread shared-memory stash by cp.async before the ring
-// wait, so they arrive during the stencil instead of after it: 9 floats a
-// thread (the auxiliary values), 18 (and the RK sum) or 27 (and the step
-// start); 0: none.  Measured on 400 x 400 x 200: 32 x 8 tiles 7.97 ms per
-// step without, 7.57 with 9, 8.30 with 18 (the larger carve-out leaves L1
-// too small for the point loads); 32 x 4 tiles 8.03 without, 7.98 with 27.
-#ifndef CG_PML_STASH
-#define CG_PML_STASH (TY == 8 ? 9 : 27)
-#endif
-// 1: the first face's operands the stash does not hold are prefetched into
-// L2 with the stash copies (32 x 8 tiles: 7.57 -> 7.51 ms per step; loading
-// them into registers there instead spilled and took 9.26 ms)
-#ifndef CG_PML_REST_PREFETCH
-#define CG_PML_REST_PREFETCH 1
-#endif
-#define STASH_F (CG_PML_STASH * CW)
-// the same stash in the ring pipeline (batches, linked parts), FP32 only:
-// 9 floats took a 400x400x200 ring session from 8.25 to 8.04 ms per step but
-// batch32 from 34.6 to 35.5 ms (its small shots' L1 shrinks with the
-// carve-out), and batches are the ring's main users, so none by default
-#ifndef CG_PML_STASH_RING
-#define CG_PML_STASH_RING 0
-#endif
-#define STASH_RING_F (CG_PML_STASH_RING * TX * TY)
 #define SLOT_HB (9 * PF * 2)  // mixed storage: bytes of a slot's FP16 delta box
 // Mixed storage: the ring also holds each plane's FP16 delta box, so a CTA
 // needs 104 KB and two fit on an SM.
@@ -192,21 +174,12 @@ static_assert(SLOT_SF % 32 == 0 && CSLOT_SF % 32 == 0 && SLOT_HSF % 64 == 0 && C
 
 static size_t stage_smem(bool mix)
 {
-    return (size_t)NSLOT * (SLOT_SF * 4 + (mix ? SLOT_HSF * 2 : 0)) + (mix ? 0 : STASH_RING_F * 4) + NSLOT * 8;
+    return (size_t)NSLOT * (SLOT_SF * 4 + (mix ? SLOT_HSF * 2 : 0)) + NSLOT * 8;
 }
 static size_t stage2_smem()
 {
-    return (size_t)(NHSLOT * SLOT_SF + NCSLOT * CSLOT_SF + STASH_F) * 4 + (NHSLOT + NCSLOT) * 8;
+    return (size_t)(NHSLOT * SLOT_SF + NCSLOT * CSLOT_SF) * 4 + (NHSLOT + NCSLOT) * 8;
 }
-
-// one float from global to shared memory, asynchronously (cp.async); this
-// thread waits for its own copies with cp_async_wait_all
-__device__ __forceinline__ void cp_async4(float *dst, const float *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Stencil taps: hc points at this thread's cell of the current plane's halo
 // box (x and y derivatives), zp[m] at its cell of plane k + FB3*(m-1) for the
@@ -399,13 +372,10 @@ __device__ __forceinline__ __half to_h16(float x, float sc)
 // delta into the FP32 box in place, so the taps read the stage's input as in
 // the FP32 kernel.
 //
-// V2 = true: the split pipeline (see CSLOT_F above).  Only the current plane
-// needs its x/y halo; the other planes of the z window need only the tile's
-// interior columns, so the shared memory left over holds the current plane's
-// point operands, brought in by TMA during the previous plane instead of
-// being loaded by every thread at the plane's start.
+// V2 = true: the split pipeline (see CSLOT_F above).
 //
-// IRK >= 0: the RK stage at compile time (the split pipeline), -1: a.irk.
+// IRK >= 0: the RK stage at compile time (a runtime stage spilled 200-300
+// bytes a thread), -1: a.irk (batches with FP16 storage).
 template <int FB1, int FB2, int FB3, bool BATCH, bool HOUT, bool MIX = false, bool V2 = false, int IRK = -1>
 __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                                             : V2 ? CG_SPLIT_CTAS_PER_SM
@@ -418,15 +388,10 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
     float *ring = reinterpret_cast<float *>(smem_raw);   // V2: the halo ring (2 slots)
     __half *ring16 = reinterpret_cast<__half *>(smem_raw + NSLOT * SLOT_SF * 4);
     float *col = ring + NHSLOT * SLOT_SF;                 // V2: column ring
-    // PML operands of the first face (split: after the column ring; ring:
-    // after the ring)
-    float *stash = V2 ? col + NCSLOT * CSLOT_SF : ring + NSLOT * SLOT_SF;
     constexpr int NCS = V2 ? NCSLOT : NSLOT;              // column (V2) or ring slots
-    constexpr int NSTASH = V2 ? CG_PML_STASH : MIX ? 0 : CG_PML_STASH_RING;
-    constexpr bool STASH = NSTASH > 0;
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(
-        V2 ? smem_raw + (NHSLOT * SLOT_SF + NCSLOT * CSLOT_SF + STASH_F) * 4
-           : smem_raw + NSLOT * (SLOT_SF * 4 + (MIX ? SLOT_HSF * 2 : 0)) + (MIX ? 0 : STASH_RING_F * 4));
+        V2 ? smem_raw + (NHSLOT * SLOT_SF + NCSLOT * CSLOT_SF) * 4
+           : smem_raw + NSLOT * (SLOT_SF * 4 + (MIX ? SLOT_HSF * 2 : 0)));
     // barrier of column (V2) or ring slot s
     auto cbar = [&](int s) -> unsigned long long * { return V2 ? &bars[NHSLOT + s] : &bars[s]; };
     __shared__ int s_abort, s_item;
@@ -723,38 +688,6 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                     for (int f = 0; f < 9; f++) tv[f] = CG_LD(a.Wb[f * F + q]), cv[f] = CG_LD(a.Wc[f * F + q]);
             }
         }
-        // the first PML face of this point: its operands into the stash
-        int fc0 = -1;
-        if constexpr (STASH) {
-            const bool inz1p = (a.pml_on & 4) && k < CGFDM_HALO + nPML;
-            fc0 = !active ? -1 : inx1 ? 0 : iny1 ? 1 : inz1p ? 2 : inx2 ? 3 : iny2 ? 4 : -1;
-            if (fc0 >= 0) {
-                const PmlFace &P = a.face[fc0];
-                const long long pos = pml_pos(fc0, i, j, k);
-                float *st = stash + ty * TX + tx;
-                const float *cur = pml_in(P);
-                // the values its RK update reads beside them (see pml_in)
-                const float *o1 = CG_RK_SUM ? (irk != 0 ? P.T : nullptr) : irk == 3 ? P.B : nullptr;
-                const float *o2 = (CG_RK_SUM ? irk == 1 || irk == 2 : irk != 0) ? P.A : nullptr;
-                for (int f = 0; f < 9; f++) cp_async4(st + f * CW, cur + f * P.count + pos);
-                if (NSTASH >= 18 && o1)
-                    for (int f = 0; f < 9; f++) cp_async4(st + (9 + f) * CW, o1 + f * P.count + pos);
-                if (NSTASH >= 27 && o2)
-                    for (int f = 0; f < 9; f++) cp_async4(st + (18 + f) * CW, o2 + f * P.count + pos);
-                if (NSTASH >= 36 && !CG_RK_SUM && irk == 3)
-                    for (int f = 0; f < 9; f++) cp_async4(st + (27 + f) * CW, P.C + f * P.count + pos);
-                cp_async_commit();
-                // the face's other operands (RK sum, step start, C) into L2
-                if (CG_PML_REST_PREFETCH) {
-                    if (NSTASH < 18 && o1)
-                        for (int f = 0; f < 9; f++) l2_prefetch(o1 + f * P.count + pos);
-                    if (NSTASH < 27 && o2)
-                        for (int f = 0; f < 9; f++) l2_prefetch(o2 + f * P.count + pos);
-                    if (NSTASH < 36 && !CG_RK_SUM && irk == 3)
-                        for (int f = 0; f < 9; f++) l2_prefetch(P.C + f * P.count + pos);
-                }
-            }
-        }
         const int kk_new = k - za + 4;
         bool okw = mbar_wait_bounded(smem_u32(cbar(slot_of(kk_new))), parity_of(kk_new), wlim);
         if constexpr (V2) {
@@ -810,6 +743,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
             // the scale of each direction's differences goes into its metric
             // row, the medium and DT onto the sums over the directions: about
             // 160 operations a point where the reference's order takes 330
+            // (400x400x200, with the zero metric terms: 8.2 -> 7.4 ms per step)
             const float mx = xi_x * (FB1 * rDH * bx), my = et_y * (FB2 * rDH * by), sz = FB3 * rDH * bz;
             const float m0 = zt_x * sz, m1 = zt_y * sz, m2 = zt_z * sz;
             float e0, e1, e2;
@@ -926,25 +860,22 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
             // every operand of this face loaded before the first store: the
             // stores go through pointers the compiler cannot tell apart from
             // the loads, which would otherwise wait for them (8.24 ms per
-            // step on 400x400x200 against 8.02 with them first)
+            // step on 400x400x200 against 8.02 with them first).  Copying them
+            // to shared memory during the stencil took more L1 from the point
+            // loads than it hid: 64x60x48 0.127 ms per step with 27 floats a
+            // thread, 0.108 without, 213x151x117 0.947 and 0.893.
             float xa[9], xt[9], xc[9];
-            const bool st_ = STASH && fc == fc0;
-            const float *st = stash + ty * TX + tx;
-            if (st_) cp_async_wait_all();
 #pragma unroll
-            for (int f = 0; f < 9; f++) aux[f] = !on(f) ? 0.0f : st_ ? st[f * CW] : cur[f * P.count + pos];
+            for (int f = 0; f < 9; f++) aux[f] = on(f) ? cur[f * P.count + pos] : 0.0f;
             if (need_t)
 #pragma unroll
-                for (int f = 0; f < 9; f++)
-                    xt[f] = !on(f) ? 0.0f : st_ && NSTASH >= 18 ? st[(9 + f) * CW] : pt[f * P.count + pos];
+                for (int f = 0; f < 9; f++) xt[f] = on(f) ? pt[f * P.count + pos] : 0.0f;
             if (need_a)
 #pragma unroll
-                for (int f = 0; f < 9; f++)
-                    xa[f] = !on(f) ? 0.0f : st_ && NSTASH >= 27 ? st[(18 + f) * CW] : P.A[f * P.count + pos];
+                for (int f = 0; f < 9; f++) xa[f] = on(f) ? P.A[f * P.count + pos] : 0.0f;
             if (!SUM && irk == 3)
 #pragma unroll
-                for (int f = 0; f < 9; f++)
-                    xc[f] = !on(f) ? 0.0f : st_ && NSTASH >= 36 ? st[(27 + f) * CW] : P.C[f * P.count + pos];
+                for (int f = 0; f < 9; f++) xc[f] = on(f) ? P.C[f * P.count + pos] : 0.0f;
 #pragma unroll
             for (int f = 0; f < 9; f++) hA[f] = (rhs[f] - alpha_d * aux[f]) * DT;
             if (DIR < 2 && surf) {
@@ -1119,9 +1050,6 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
         }
         break;
     }
-    // no copy into the stash outlives the item (one may be pending after a
-    // failed wait)
-    if constexpr (STASH) cp_async_wait_all();
     seq0 += (unsigned)(issued - kf + 1);
     hseq0 += (unsigned)(ke - kb);
     }  // work items

@@ -46,10 +46,6 @@ __device__ __forceinline__ void tma_load_4d(unsigned dst, const void *tmap, int 
         : "memory");
 }
 
-__device__ __forceinline__ void l2_prefetch(const void *p)
-{
-    asm volatile("prefetch.global.L2 [%0];\n" ::"l"((unsigned long long)p));
-}
 __device__ __forceinline__ void tma_prefetch_4d(const void *tmap, int x, int y, int z, int f)
 {
     asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(

@@ -10,6 +10,8 @@ run's FP32 form.  Sizes sit at the edges of tiles and of the pencils, with
 absorbing layers that overlap at the smallest ones.
 """
 
+import json
+
 import numpy as np
 import pytest
 
@@ -80,3 +82,48 @@ def test_stage_matches_all_terms_run_bit_for_bit(tmp_path, nx, ny, nz, nPML, gri
         np.testing.assert_array_equal(W_p.astype(np.float32), s.wavefield())
         np.testing.assert_array_equal(st_p.astype(np.float32), s.stations())
         np.testing.assert_array_equal(pgv_p.astype(np.float32), s.pgv()[:, :, :2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("options", ['{}', '{"stagePipeline": "ring"}'])
+@pytest.mark.parametrize("nx,ny,nz,nPML,grid", [(33, 9, 17, 4, "hill"), (13, 41, 19, 8, "file"), (66, 11, 25, 6, "flat")])
+def test_default_build_stays_as_close_to_fp64(tmp_path, nx, ny, nz, nPML, grid, options):
+    """The default build ends a step from its three stage values instead of a
+    running sum and factors the sums: no further from the FP64 run than twice
+    the exact build, with a source whose cube reaches into the halo (those
+    cells are held in all four stage buffers)."""
+    d = _case(nx, ny, nz, nPML, grid, 17, tmp_path)
+    p = tmp_path / f"{grid}_{nx}x{ny}x{nz}_CGFDM" / "params.json"
+    q = json.loads(p.read_text())
+    q.update(sourceX=1, sourceY=2)
+    p.write_text(json.dumps(q))
+    err = {}
+    for flavor in ("exact", "fast"):
+        with Session(d, options=options, flavor=flavor) as s:
+            st64, _, W64 = s.run_precise(17, bits=64, wavefield=True)
+            s.run(17)
+            W, st = s.wavefield(), s.stations()
+        err[flavor] = max(pu.rel_l2(W[..., :3], W64[..., :3]), pu.rel_l2(W[..., 3:], W64[..., 3:]),
+                          pu.rel_l2(st, st64))
+    assert err["exact"] < 1e-5
+    assert err["fast"] <= 2 * err["exact"] + 1e-7
+
+
+@pytest.mark.gpu
+def test_halo_of_an_initial_wavefield_is_held_in_every_stage(tmp_path):
+    """set_wavefield keeps its halo through all stages: the default build
+    (four stage buffers) and the exact one (three) agree, 1e-6 over nine steps
+    of about ten roundings each."""
+    d = _case(33, 21, 17, 4, "hill", 9, tmp_path)
+    out = {}
+    for flavor in ("exact", "fast"):
+        with Session(d, flavor=flavor) as s:
+            i = s.info
+            rng = np.random.default_rng(4)
+            w = _waves((i.nzp, i.nyp, i.nxp), 4, [0.05] * 3 + [5e5] * 6)
+            w[:, :3] = w[:, 3:6] + rng.normal(size=w[:, :3].shape) * w.std(axis=(0, 1, 2)) * 0.1
+            s.set_wavefield(w.astype(np.float32))
+            s.run(9)
+            out[flavor] = s.wavefield()
+    for part in (slice(0, 3), slice(3, 9)):
+        assert pu.rel_l2(out["fast"][..., part], out["exact"][..., part]) <= 1e-6
