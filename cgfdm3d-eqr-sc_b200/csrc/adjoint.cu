@@ -298,6 +298,9 @@ __device__ __forceinline__ float tap_sum(const float *__restrict__ f, long long 
     return s;
 }
 
+// The FB signs are template parameters: the x taps become fixed offsets from
+// one address.
+template <int FB1, int FB2, int FB3>
 __global__ void ADJ_BOUNDS_GATHER k_adj_gather(const __grid_constant__ AdjStageArgs a)
 {
     const DevGrid g = a.g;
@@ -308,7 +311,6 @@ __global__ void ADJ_BOUNDS_GATHER k_adj_gather(const __grid_constant__ AdjStageA
     if (i >= _nx || j >= _ny) return;
     const long long F = g.fstride, q = g.at(i, j, k), s = g.at2(i, j), P = g.plane;
     const float rDH = a.rDH, DT = a.DT;
-    const int FB1 = a.FB1, FB2 = a.FB2, FB3 = a.FB3;
 
     float nu[9];
 #pragma unroll
@@ -436,7 +438,16 @@ cudaError_t launch_adj_stage(const AdjStageArgs &a, cudaStream_t st)
     dim3 b(32, ADJ_TY), gr((a.g.nx + 31) / 32, (a.g.ny + ADJ_TY - 1) / ADJ_TY, a.g.nz);
     k_adj_pre<<<gr, b, 0, st>>>(a);
     CUDA_TRY(cudaGetLastError());
-    k_adj_gather<<<gr, b, 0, st>>>(a);
+    switch ((a.FB1 > 0) * 4 + (a.FB2 > 0) * 2 + (a.FB3 > 0)) {
+    case 0: k_adj_gather<-1, -1, -1><<<gr, b, 0, st>>>(a); break;
+    case 1: k_adj_gather<-1, -1, 1><<<gr, b, 0, st>>>(a); break;
+    case 2: k_adj_gather<-1, 1, -1><<<gr, b, 0, st>>>(a); break;
+    case 3: k_adj_gather<-1, 1, 1><<<gr, b, 0, st>>>(a); break;
+    case 4: k_adj_gather<1, -1, -1><<<gr, b, 0, st>>>(a); break;
+    case 5: k_adj_gather<1, -1, 1><<<gr, b, 0, st>>>(a); break;
+    case 6: k_adj_gather<1, 1, -1><<<gr, b, 0, st>>>(a); break;
+    default: k_adj_gather<1, 1, 1><<<gr, b, 0, st>>>(a); break;
+    }
     return cudaGetLastError();
 }
 
