@@ -79,9 +79,8 @@ __device__ __forceinline__ F2 operator-(F2 a, F2 b) { return vsub(a, b); }
 __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return vmul(a, b); }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return vfma(a, b, c); }
 // (ftz: one instruction where the subnormal-safe form takes a compare, a
-// select and two multiplications; the arguments are squared indicators of at
-// least 8e-13 and sums of their reciprocals, subnormal only for differences
-// beyond 2e9 between neighbouring cells)
+// select and two multiplications; weno_pair scales the arguments, so that no
+// finite square of an indicator leads to a subnormal one)
 __device__ __forceinline__ F2 rcp2(F2 x)
 {
     float a, b;
@@ -117,7 +116,13 @@ __device__ __forceinline__ void weno_pair(F2 a, F2 b, F2 c, F2 d, F2 e, F2 &uL, 
     const F2 B0 = fma2(s0, s0, fma2(k * t0, t0, eps));
     const F2 B1 = fma2(s1, s1, fma2(k * t1, t1, eps));
     const F2 B2 = fma2(n2, n2, fma2(k * t2, t2, eps));
-    const F2 r0 = rcp2(B0 * B0), r1 = rcp2(B1 * B1), r2 = rcp2(B2 * B2);
+    // the squares scaled by 2^-60 (which cancels in the weights): between
+    // 7e-31 and the 8e37 past which the reciprocal would be flushed to zero
+    // and the weights 0/0 lie indicators up to 1e28.  Unscaled, indicators of
+    // 9e18 were flushed (differences of 3e9 between neighbouring cells) where
+    // squares in FP32 hold to 1.8e19.
+    const F2 sc = pk(0x1p-60f);
+    const F2 r0 = rcp2((sc * B0) * B0), r1 = rcp2((sc * B1) * B1), r2 = rcp2((sc * B2) * B2);
     const F2 wm = two * r1, far0 = fifth * r0, far2 = fifth * r2;
     // q of the face-side, centred and far sub-stencils
     const F2 nL = fma2(r2, fma2(four, d2, n2), fma2(wm, fma2(three, d2, d1), far0 * fma2(two, t0, s0)));

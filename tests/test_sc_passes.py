@@ -47,3 +47,38 @@ def test_passes_match_fp64(tmp_path, nx, ny, nz, source):
                           pu.rel_l2(st[..., :3], st64[..., :3]), pu.rel_l2(st[..., 3:], st64[..., 3:]))
     print(f"{nx}x{ny}x{nz} {source}: fast {err['fast']:.2e}, exact {err['exact']:.2e}")
     assert err["fast"] <= 2 * err["exact"] + 1e-7
+
+
+def _waves(shape, amp, rng):
+    z, y, x = np.meshgrid(*[np.arange(n) for n in shape], indexing="ij")
+    w = np.zeros(shape + (9,))
+    for f in range(9):
+        for _ in range(4):
+            k = rng.normal(size=3)
+            k *= 2 * np.pi / (np.linalg.norm(k) * rng.uniform(8, 20))
+            w[..., f] += amp[f] * rng.normal() * np.cos(k[0] * x + k[1] * y + k[2] * z + rng.uniform(0, 6.3))
+    return w.astype(np.float32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift", [1, 2, 3, 8, 16])
+def test_passes_scale_with_the_field(tmp_path, shift):
+    """The scheme is homogeneous but for the 1e-6 in the smoothness indicators:
+    a field 2^shift times as large stays finite and gives 2^shift times the
+    result.  Momentum of 5e8 gives indicators of 1e16 to 1e17; three more
+    powers of two take them past 9e18, where the reciprocal of an unscaled
+    square is subnormal.  Strains of 40 have indicators of 1 at least almost
+    everywhere, so the 1e-6 moves a weight by 1e-6 there; the states' spread
+    over the sub-stencils is a tenth of the field or less."""
+    d = _run(37, 29, 31, "ricker", tmp_path)
+    out = []
+    with Session(d) as s:
+        i = s.info
+        w = _waves((i.nzp, i.nyp, i.nxp), [5e8] * 3 + [40.0] * 6, np.random.default_rng(3))
+        for n in (0, shift):
+            s.set_wavefield(w * np.float32(2.0**n))
+            s.run(1)
+            out.append(s.wavefield().astype(np.float64) / 2.0**n)
+    assert np.isfinite(out[1]).all()
+    for part in (slice(0, 3), slice(3, 9)):
+        assert pu.rel_l2(out[1][..., part], out[0][..., part]) <= 1e-6
