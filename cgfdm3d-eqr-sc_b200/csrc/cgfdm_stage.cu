@@ -65,10 +65,12 @@
 #endif
 // RK4 without the running sum: the step ends from the step start and the
 // three stage values, m + ((B - m) + 2 (C - m) + (D - m)) / 3 + h3 / 6, each in
-// a buffer of its own.  A step then moves 149 floats a point instead of 176
-// and 117 an absorbing-layer point instead of 144, and rounds less (the
-// differences are exact where the stages are close).  The exact build keeps
-// the reference's running sum T.
+// a buffer of its own.  A step then moves 149 floats a point instead of 176,
+// and rounds less (the differences are exact where the stages are close).  The
+// absorbing layers' auxiliaries, which no other point reads, need three
+// buffers: stage 1 stores C over T and (B - m) + 2 (C - m) over B, stage 2 D
+// over C, 117 floats a point instead of 144 (18 + 36 + 27 + 36).  The exact
+// build keeps the reference's running sum T.
 #ifdef CGFDM_EXACT
 #define CG_RK_SUM 1
 #else
@@ -337,16 +339,21 @@ __device__ __forceinline__ void ljt_z_m(const MixIn &w, const float *__restrict_
     for (int c = 0; c < 3; c++) out[c] = lop(J[0][c], J[1][c], J[2][c], J[3][c], J[4][c], FB, rDH);
 }
 
-// RK4 without the running sum: stage irk's value (irk 0..2) and the step's
-// end from the step start m and the stage values b, c, d.  Every rounding is
-// explicit, so the pipelines agree bit for bit.
+// RK4 without the running sum: stage irk's value (irk 0..2), the sum of the
+// first two stages' differences and the step's end from the step start m, that
+// sum bc and the last stage value d.  Every rounding is explicit, so the
+// pipelines agree bit for bit.
 __device__ __forceinline__ float rk_stage(int irk, float m, float h)
 {
     return irk == 2 ? __fadd_rn(m, h) : __fmaf_rn(RK_ALPHA2, h, m);
 }
-__device__ __forceinline__ float rk_end(float m, float b, float c, float d, float h)
+__device__ __forceinline__ float rk_bc(float m, float b, float c)
 {
-    const float s = __fadd_rn(__fmaf_rn(2.0f, __fsub_rn(c, m), __fsub_rn(b, m)), __fsub_rn(d, m));
+    return __fmaf_rn(2.0f, __fsub_rn(c, m), __fsub_rn(b, m));
+}
+__device__ __forceinline__ float rk_end(float m, float bc, float d, float h)
+{
+    const float s = __fadd_rn(bc, __fsub_rn(d, m));
     return __fadd_rn(m, __fmaf_rn(RK_BETA4, h, __fmul_rn(RK_BETA2, s)));
 }
 
@@ -521,10 +528,10 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
         return (long long)ip + (long long)jp * g.nx + (long long)kp * g.nx * g.ny;
     };
     // a face's auxiliaries at the stage's input: A, then B B B with a running
-    // sum in T, or B C T (the three stage values) without
+    // sum in T, or B T T without
     auto pml_in = [&](const PmlFace &P) -> const float * {
         if (CG_RK_SUM) return irk == 0 ? P.A : P.B;
-        return irk == 0 ? P.A : irk == 1 ? P.B : irk == 2 ? P.C : P.T;
+        return irk == 0 ? P.A : irk == 1 ? P.B : P.T;
     };
     const int item = BATCH ? gitem - item_start[sess] : V2 ? gitem / sweeps : gitem;
     const int sweep = V2 ? gitem - item * sweeps : 0;
@@ -855,7 +862,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
             const float *cur = pml_in(P);
             constexpr bool SUM = CG_RK_SUM;
             const bool need_a = SUM ? irk == 1 || irk == 2 : irk != 0;   // the step start
-            const bool need_t = SUM ? irk != 0 : irk == 3;               // the running sum, or B
+            const bool need_t = SUM ? irk != 0 : irk == 3;               // the running sum, or that of stages 0, 1
             const float *pt = SUM ? P.T : P.B;
             // every operand of this face loaded before the first store: the
             // stores go through pointers the compiler cannot tell apart from
@@ -864,7 +871,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
             // to shared memory during the stencil took more L1 from the point
             // loads than it hid: 64x60x48 0.127 ms per step with 27 floats a
             // thread, 0.108 without, 213x151x117 0.947 and 0.893.
-            float xa[9], xt[9], xc[9];
+            float xa[9], xt[9];
 #pragma unroll
             for (int f = 0; f < 9; f++) aux[f] = on(f) ? cur[f * P.count + pos] : 0.0f;
             if (need_t)
@@ -873,9 +880,6 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
             if (need_a)
 #pragma unroll
                 for (int f = 0; f < 9; f++) xa[f] = on(f) ? P.A[f * P.count + pos] : 0.0f;
-            if (!SUM && irk == 3)
-#pragma unroll
-                for (int f = 0; f < 9; f++) xc[f] = on(f) ? P.C[f * P.count + pos] : 0.0f;
 #pragma unroll
             for (int f = 0; f < 9; f++) hA[f] = (rhs[f] - alpha_d * aux[f]) * DT;
             if (DIR < 2 && surf) {
@@ -913,13 +917,15 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
                     if (on(f)) CG_PST(P.A[f * P.count + pos], xt[f] + RK_BETA4 * hA[f]);
             }
 #else
-            float *out = irk == 0 ? P.B : irk == 1 ? P.C : irk == 2 ? P.T : P.A;
+            float *out = irk == 0 ? P.B : irk == 3 ? P.A : P.T;
 #pragma unroll
             for (int f = 0; f < 9; f++) {
                 if (!on(f)) continue;
-                CG_PST(out[f * P.count + pos], irk == 0   ? rk_stage(0, aux[f], hA[f])
-                                               : irk == 3 ? rk_end(xa[f], xt[f], xc[f], aux[f], hA[f])
-                                                          : rk_stage(irk, xa[f], hA[f]));
+                const float v = irk == 0   ? rk_stage(0, aux[f], hA[f])
+                                : irk == 3 ? rk_end(xa[f], xt[f], aux[f], hA[f])
+                                           : rk_stage(irk, xa[f], hA[f]);
+                CG_PST(out[f * P.count + pos], v);
+                if (irk == 1) CG_PST(P.B[f * P.count + pos], rk_bc(xa[f], aux[f], v));
             }
 #endif
         };
@@ -998,7 +1004,7 @@ __global__ void __launch_bounds__(TX *TY, MIX  ? CG_MIX_CTAS_PER_SM
 #else
 #pragma unroll
         for (int f = 0; f < 9; f++)
-            wout[f] = irk == 3 ? rk_end(mv[f], tv[f], cv[f], T.c(f), h[f]) : rk_stage(irk, mv[f], h[f]);
+            wout[f] = irk == 3 ? rk_end(mv[f], rk_bc(mv[f], tv[f], cv[f]), T.c(f), h[f]) : rk_stage(irk, mv[f], h[f]);
 #endif
 #pragma unroll
         for (int f = 0; f < 9; f++) CG_ST(a.Wout[f * F + q], wout[f]);

@@ -154,7 +154,6 @@ int Session::set_medium(const float *host)
             CU(cudaMemsetAsync(face_[fc].A, 0, b, stream));
             CU(cudaMemsetAsync(face_[fc].B, 0, b, stream));
             CU(cudaMemsetAsync(face_[fc].T, 0, b, stream));
-            if (face_[fc].C) CU(cudaMemsetAsync(face_[fc].C, 0, b, stream));
         }
     CU(cudaMemsetAsync(pgv_, 0, sizeof(float) * m.g.nx * m.g.ny * 2, stream));
     if (pga_) CU(cudaMemsetAsync(pga_, 0, sizeof(float) * m.g.nx * m.g.ny * 2, stream));

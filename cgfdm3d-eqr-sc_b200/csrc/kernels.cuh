@@ -21,10 +21,11 @@ cudaError_t launch_scale_moment(float *rate, const long long *cell, long long np
 // ------------------------------------------------------------ PML state
 // One absorbing face: Aux fields for its slab, each buffer 9 fields of
 // `count` floats.  A holds the step-start value and receives the final stage;
-// B, C and T the values of stages 0, 1 and 2 or, in the exact build, B every
-// stage's and T the RK accumulator (no C).
+// B holds stage 0's value and from stage 1 on the sum of the differences of
+// stages 0 and 1, T the values of stages 1 and 2.  In the exact build B holds
+// every stage's value and T the RK accumulator.
 struct PmlFace {
-    float *A, *B, *T, *C;
+    float *A, *B, *T;
     long long count;     // points in the slab
     int n0, n1;          // slab extent along its two fastest axes (see pml_pos)
 };

@@ -237,7 +237,7 @@ size_t Session::arena_estimate() const
                                    nP * G.nx * G.nz};
             for (int fc = 0; fc < 5; fc++)
                 if (pml_faces() & (1 << fc))
-                    for (int x = 0; x < (RK_SUM ? 3 : 4); x++) add(sizeof(float) * cnt[fc] * 9);
+                    for (int x = 0; x < 3; x++) add(sizeof(float) * cnt[fc] * 9);
         }
     }
     add(sizeof(float) * (size_t)G.nx * G.ny * 2);
@@ -426,7 +426,6 @@ int Session::setup_device()
             ALLOC(face_[fc].A, float, cnt[fc] * 9);
             ALLOC(face_[fc].B, float, cnt[fc] * 9);
             ALLOC(face_[fc].T, float, cnt[fc] * 9);
-            if (!RK_SUM) ALLOC(face_[fc].C, float, cnt[fc] * 9);
         }
     } else if (cg) {
         // PML off: unit stretching, zero damping
@@ -985,7 +984,7 @@ double Session::algo_bytes_per_step() const
     if (m.p.scheme == SCHEME_SCFDM) return 4.0 * 111.0 * n;
     if (m.p.pml) faces = (double)G.nPML * (2.0 * G.ny * G.nz + 2.0 * G.nx * G.nz + (double)G.nx * G.ny);
     // an absorbing-layer point's auxiliaries: 27 + 45 + 45 + 27 fields with a
-    // running sum, 18 + 27 + 27 + 45 without
+    // running sum, 18 + 36 + 27 + 36 without
     const double aux = 4.0 * (RK_SUM ? 144.0 : 117.0) * faces;
     // FP16 storage: 4-byte state and eight metric fields, 2-byte deltas; stage
     // 0 reads A and the metric and writes the delta (68 + 18 B), stage 1 adds

@@ -127,3 +127,16 @@ def test_halo_of_an_initial_wavefield_is_held_in_every_stage(tmp_path):
             out[flavor] = s.wavefield()
     for part in (slice(0, 3), slice(3, 9)):
         assert pu.rel_l2(out["fast"][..., part], out["exact"][..., part]) <= 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("options", [None, '{"storage": "fp16"}', '{"PML": 0}'])
+def test_default_build_needs_no_more_memory(tmp_path, options):
+    """The default build's other RK form holds as much on the device as the
+    exact build's running sum, absorbing layers included."""
+    d = _case(37, 29, 23, 6, "hill", 8, tmp_path)
+    held = {}
+    for flavor in ("exact", "fast"):
+        with Session(d, options=options, flavor=flavor) as s:
+            held[flavor] = s.info.device_bytes
+    assert held["fast"] == held["exact"] > 0
