@@ -188,11 +188,7 @@ int Batch::set_tiling(int kc, int ctas)
         err = "kchunk and ctas must be >= 1";
         return ST_ARG;
     }
-    for (Session *x : s)
-        if (int st = x->set_tiling(kc, 1 << 30)) {
-            err = x->err;
-            return st;
-        }
+    std::fill(kchunk_.begin(), kchunk_.end(), kc);
     want_ctas_ = ctas;
     if (int st = build_tables()) return st;
     drop_graph();
@@ -251,8 +247,7 @@ int Batch::autotune(int trial, int *best_kc, int *best_ctas, float *best_ms)
     // the current decomposition (each session's own pencil) first; a
     // uniform one replaces it only when faster by more than the trials'
     // noise (1 %)
-    std::vector<int> k_orig;
-    for (Session *x : s) k_orig.push_back(x->kchunk());
+    const std::vector<int> k_orig = kchunk_;
     const int want_orig = want_ctas_, t_orig = tile_;
     float ms0 = 0.0f;
     if (int st = load_all()) return st;
@@ -280,11 +275,7 @@ int Batch::autotune(int trial, int *best_kc, int *best_ctas, float *best_ms)
     }
     if (bms > 0.99f * ms0) {
         if (int st = set_tile(t_orig)) return st;
-        for (size_t i = 0; i < s.size(); i++)
-            if (int st = s[i]->set_tiling(k_orig[i], 1 << 30)) {
-                err = s[i]->err;
-                return st;
-            }
+        kchunk_ = k_orig;
         want_ctas_ = want_orig;
         if (int st = build_tables()) return st;
         drop_graph();

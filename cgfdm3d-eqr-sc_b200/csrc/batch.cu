@@ -81,31 +81,20 @@ int Batch::create(const std::vector<Session *> &sessions)
     BCU(cudaSetDevice(device));
     for (Session *x : s) BCU(cudaStreamSynchronize(x->stream));
     // the batched launch runs the ring kernel, 32 x 4 tiles unless set_tile
-    // chooses 8 rows
-    for (Session *x : s)
-        if (int st = x->set_tile(tile_)) {
-            err = x->err;
-            return st;
-        }
-    // one pencil length for the shared launch, from the tiles of all sessions
-    // (a small session's own is shorter); a session whose pencil was chosen
-    // by set_tiling or the autotuner keeps it
+    // chooses 8 rows.  One pencil length for the shared launch, from the tiles
+    // of all sessions (a small session's own is shorter); a session whose
+    // pencil was chosen by set_tiling or the autotuner brings it along
     {
         int nz = 1, sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         long long columns = 0;
         for (Session *x : s) {
             nz = std::max(nz, x->m.g.nz);
-            columns += (long long)x->stage_tiles() * x->m.g.nz;
+            columns += (long long)((x->m.g.nx + 31) / 32) * ((x->m.g.ny + tile_ - 1) / tile_) * x->m.g.nz;
         }
         const int per_sm = mix_ ? cg_stage_mix_ctas_per_sm() : cg_stage_ctas_per_sm();
         const int k = stage_chunk((columns + nz - 1) / nz, nz, sms * per_sm);
-        for (Session *x : s)
-            if (!x->tiling_chosen())
-                if (int st = x->apply_tiling(k, 1 << 30)) {
-                    err = x->err;
-                    return st;
-                }
+        for (Session *x : s) kchunk_.push_back(x->tiling_chosen() ? x->kchunk() : k);
     }
     BCU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     BCU(cudaEventCreate(&ev_[0]));
@@ -129,16 +118,25 @@ int Batch::build_tables()
 {
     const int n = (int)s.size();
     std::vector<int> items(n + 1, 0);
-    for (int i = 0; i < n; i++) items[i + 1] = items[i] + s[i]->stage_items();
+    for (int i = 0; i < n; i++) {
+        const BatchTiling t = tiling(i);
+        items[i + 1] = items[i] + s[i]->stage_items(&t);
+    }
     std::vector<CgStageDesc> d(n);
     for (int irk = 0; irk < 4; irk++) {
-        for (int i = 0; i < n; i++) s[i]->stage_desc(irk, d[i], true);
+        for (int i = 0; i < n; i++) {
+            const BatchTiling t = tiling(i);
+            s[i]->stage_desc(irk, d[i], &t);
+        }
         BCU(cudaMemcpy(desc_[irk], d.data(), sizeof(CgStageDesc) * n, cudaMemcpyHostToDevice));
     }
     if (mix_)
         for (int par = 0; par < 2; par++)
             for (int irk = 0; irk < 4; irk++) {
-                for (int i = 0; i < n; i++) s[i]->stage_desc_mix(par, irk, d[i]);
+                for (int i = 0; i < n; i++) {
+                    const BatchTiling t = tiling(i);
+                    s[i]->stage_desc_mix(par, irk, d[i], &t);
+                }
                 BCU(cudaMemcpy(descm_[par][irk], d.data(), sizeof(CgStageDesc) * n, cudaMemcpyHostToDevice));
             }
     BCU(cudaMemcpy(items_, items.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
@@ -156,14 +154,14 @@ int Batch::set_tile(int rows)
         err = "stage tiles have 4 or 8 rows";
         return ST_ARG;
     }
+    for (Session *x : s)
+        if (rows == 8 && (x->mixed() || x->part_session_)) {
+            err = "32 x 8 stage tiles need FP32 storage and a whole grid";
+            return ST_OPTIONS;
+        }
     BCU(cudaSetDevice(device));
     for (Session *x : s) BCU(cudaStreamSynchronize(x->stream));
     BCU(cudaStreamSynchronize(stream));
-    for (Session *x : s)
-        if (int st = x->set_tile(rows)) {
-            err = x->err;
-            return st;
-        }
     tile_ = rows;
     if (int st = build_tables()) return st;
     drop_graph();

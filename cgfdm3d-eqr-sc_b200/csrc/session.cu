@@ -548,8 +548,9 @@ int stage_chunk(long long tiles, int nz, int ctas)
 
 // The four stage descriptors (RK4 stage irk reads buffer STAGE_IN[irk] and
 // writes STAGE_OUT[irk]) with their tensor maps.
-void Session::stage_desc(int irk, CgStageDesc &d, bool batched) const
+void Session::stage_desc(int irk, CgStageDesc &d, const BatchTiling *batch) const
 {
+    const int rows = batch ? batch->rows : tile_, kchunk = batch ? std::min(batch->kchunk, m.g.nz) : kchunk_;
     float *A = W_[0], *T = W_[3];
     std::memset(&d, 0, sizeof d);
     CgStageArgs &a = d.a;
@@ -571,7 +572,7 @@ void Session::stage_desc(int irk, CgStageDesc &d, bool batched) const
     a.nPML = m.g.nPML;
     a.pml_on = pml_faces();
     a.fs_on = m.fs_top ? 1 : 0;
-    a.kchunk = kchunk_;
+    a.kchunk = kchunk;
     a.rDH = m.g.rDH;
     a.DT = (float)m.p.DT;
     a.err = err_dev_;
@@ -579,10 +580,11 @@ void Session::stage_desc(int irk, CgStageDesc &d, bool batched) const
     a.stall_item = stall_item_;
     a.stall_fill = stall_fill_;
     a.wait_limit = wait_limit_;
-    a.ntiles_x = ntx_, a.ntiles_y = nty_, a.nchunk = nchunk_;
-    a.sweeps = tile_ / 4;
+    a.ntiles_x = ntx_, a.ntiles_y = (m.g.ny + rows - 1) / rows, a.nchunk = (m.g.nz + kchunk - 1) / kchunk;
+    a.sweeps = rows / 4;
     for (int f = 0; f < 6; f++) a.ho[f] = ho_[irk][f];
-    const CgStageMaps &M = (split() && !batched ? split_maps_ : maps_)[STAGE_IN[irk]];
+    // (the split pipeline sweeps an 8-row tile in two 4-row sweeps)
+    const CgStageMaps &M = maps_[rows == 8 && (batch || !split())][STAGE_IN[irk]];
     std::memcpy(d.tmW, M.win, 128);
     std::memcpy(d.tmC, M.cjm, 128);
     std::memcpy(d.tmC1, M.cjm1, 128);
@@ -593,7 +595,12 @@ void Session::stage_desc(int irk, CgStageDesc &d, bool batched) const
 }
 
 // (the split pipeline hands an item's 4-row sweeps out one by one)
-int Session::stage_items() const { return ntx_ * nty_ * nchunk_; }
+int Session::stage_items(const BatchTiling *batch) const
+{
+    if (!batch) return ntx_ * nty_ * nchunk_;
+    const int kchunk = std::min(batch->kchunk, m.g.nz);
+    return ntx_ * ((m.g.ny + batch->rows - 1) / batch->rows) * ((m.g.nz + kchunk - 1) / kchunk);
+}
 int Session::stage_units() const { return stage_items() * (split() ? tile_ / 4 : 1); }
 
 // Absorbing faces as stage-kernel bits x1 y1 z1 x2 y2 (PML off: none).
@@ -611,18 +618,16 @@ int Session::stage_ctas_per_sm() const
     return tile_ == 8 ? ty8::cg_stage_ctas_per_sm() : cg_stage_ctas_per_sm();
 }
 
-// Tensor maps of the stencil inputs: for the ring kernel (batches) boxes of
-// the tile height, for the split pipeline's own launches of its 4-row sweeps.
+// Tensor maps of the stencil inputs, with boxes of either tile height.
 int Session::build_maps()
 {
-    for (int split_set = 0; split_set < 2; split_set++) {
-        const bool eight = !split_set && tile_ == 8;
+    for (int eight = 0; eight < 2; eight++) {
         auto tmap = [&](void *out, const float *base, int nf, bool halo, int box_nf = 0) {
             return eight ? ty8::make_field_tmap(out, base, g, nf, halo, box_nf)
                          : make_field_tmap(out, base, g, nf, halo, box_nf);
         };
         for (int b = 0; b < 4; b++) {
-            CgStageMaps &M = (split_set ? split_maps_ : maps_)[b];
+            CgStageMaps &M = maps_[eight][b];
             CU(tmap(M.win, W_[b], 9, true));
             CU(tmap(M.winp, W_[b], 9, false));
             CU(tmap(M.cjm, cjm_, 13, false, 3));
@@ -651,7 +656,6 @@ int Session::set_tile(int rows)
     int dev_sms = 148;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device);
     grid_ctas_ = (int)std::min<long long>((long long)dev_sms * stage_ctas_per_sm(), (long long)stage_units());
-    if (int st = build_maps()) return st;
     if (int st = build_stage_descs()) return st;
     if (graph8_) cudaGraphExecDestroy(graph8_);
     if (graph8_src_) cudaGraphDestroy(graph8_src_);
@@ -686,9 +690,9 @@ int Session::build_stage_descs()
 // Mixed storage: stage irk of a step of the given parity.  The state A is
 // read (with the delta of the previous stage as stencil input) and, in
 // stage 3, the next state written to the other buffer; deltas go Sb -> Sc -> Sb.
-void Session::stage_desc_mix(int parity, int irk, CgStageDesc &d) const
+void Session::stage_desc_mix(int parity, int irk, CgStageDesc &d, const BatchTiling *batch) const
 {
-    stage_desc(irk, d);   // the common arguments; buffers and maps replaced below
+    stage_desc(irk, d, batch);   // the common arguments; buffers and maps replaced below
     CgStageArgs &a = d.a;
     float *A = parity ? Walt_ : W_[0], *An = parity ? W_[0] : Walt_;
     a.gh = gh_;

@@ -34,6 +34,12 @@ constexpr int STAGE_IN[4] = {0, 1, 2, 3}, STAGE_OUT[4] = {1, 2, 3, 0};
 // planes per work item of a stage launch (csrc/session.cu)
 int stage_chunk(long long tiles, int nz, int ctas);
 
+// How a batch's launch cuts a session's grid: rows of the column tiles (4 or
+// 8) and planes per work item.  The batch's own: the sessions keep theirs.
+struct BatchTiling {
+    int rows, kchunk;
+};
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -167,7 +173,7 @@ private:
     cudaGraphExec_t graph8_ = nullptr;
     cudaGraph_t graph8_src_ = nullptr;
     cudaEvent_t ev_[4] = {};
-    CgStageMaps maps_[4] = {}, split_maps_[4] = {};  // TMA descriptors per stencil input A, B, C, D
+    CgStageMaps maps_[2][4] = {};                    // TMA descriptors for 4- and 8-row tiles, per stencil input A, B, C, D
     CgStageDesc desc_host_[4] = {};                  // stage descriptors, one per RK stage
     int build_stage_descs();
     int *work_dev_ = nullptr;                        // persistent-CTA work counters
@@ -192,7 +198,7 @@ private:
     float zs_min_ = 0, zp_max_ = 0;
     CgStageDesc desc_mix_[2][4] = {};
     int tile_ = 4;
-    int build_maps();                                // tensor maps of the stencil inputs for tile_
+    int build_maps();                                // tensor maps of the stencil inputs
     int stage_ctas_per_sm() const;
     bool split() const { return m.p.stage_split && !mix_ && !part_session_; }   // the split pipeline's kernel
     int *stall_dev_ = nullptr;                       // test hook of the stage kernel's bounded waits
@@ -200,9 +206,8 @@ private:
     long long wait_limit_ = 0;
 
 public:
-    // Column-tile height of the CGFDM stage kernel (4 or 8 rows of 32), the
-    // tensor maps and work items built for it; set_tile re-encodes them
-    // (8 only with FP32 storage on a whole grid)
+    // Column-tile height of the CGFDM stage kernel (4 or 8 rows of 32; 8 only
+    // with FP32 storage on a whole grid)
     int tile() const { return tile_; }
     int set_tile(int rows);
     // one RK stage of this session's CGFDM step, with the pipeline and tile
@@ -219,13 +224,12 @@ public:
     // kernel gives up after `wait_cycles` clocks (0: the default limit).
     int test_stall(int item, int fill, long long wait_cycles);
     // the stage descriptor of RK stage irk (with FP16 storage: for the
-    // step-start state of step parity `parity`), and the stage's work items
-    // (batches use these)
-    void stage_desc(int irk, CgStageDesc &d, bool batched = false) const;
-    void stage_desc_mix(int parity, int irk, CgStageDesc &d) const;
-    int stage_items() const;
+    // step-start state of step parity `parity`), and the stage's work items;
+    // for a batch's launch cut as it says
+    void stage_desc(int irk, CgStageDesc &d, const BatchTiling *batch = nullptr) const;
+    void stage_desc_mix(int parity, int irk, CgStageDesc &d, const BatchTiling *batch = nullptr) const;
+    int stage_items(const BatchTiling *batch = nullptr) const;
     int stage_units() const;      // what the launch's counter hands out
-    int stage_tiles() const { return ntx_ * nty_; }
     int pml_faces() const;
     int launch_sources_on(cudaStream_t st);
     int launch_stations_on(cudaStream_t st);

@@ -86,3 +86,37 @@ def test_fp16_storage_batch_matches_single_runs(tmp_path):
     finally:
         for s in both:
             s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("options", [None, '{"storage": "fp16"}', '{"stagePipeline": "ring", "stageTile": 8}'])
+def test_batch_leaves_the_sessions_their_tiling(tmp_path, options):
+    """A batch cuts its shared launch in its own way; what the sessions use
+    when they run alone -- pencils and tile height -- is what it was, during
+    the batch and after it, tuned or not, and a session's chosen pencil and the
+    runs alone afterwards keep the results."""
+    dirs = _shots(tmp_path)
+    alone = []
+    for d in dirs:
+        with Session(d, options=options) as s:
+            s.run(s.info.NT)
+            alone.append((s.stations(), s.wavefield(), s.pgv()))
+    sessions = [Session(d, options=options) for d in dirs]
+    try:
+        sessions[2].set_tiling(3, 37)
+        before = [(s.tiling(), s.stage_tile()) for s in sessions]
+        with Batch(sessions) as b:
+            b.run(3)
+            if options is None or "fp16" not in options:
+                b.autotune(2)
+                b.set_stage_tile(12 - b.stage_tile())
+            b.run(4)
+            assert [(s.tiling(), s.stage_tile()) for s in sessions] == before
+        assert [(s.tiling(), s.stage_tile()) for s in sessions] == before
+        for s, ref in zip(sessions, alone):
+            s.run(100)
+            for a, r in zip((s.stations(), s.wavefield(), s.pgv()), ref):
+                np.testing.assert_array_equal(a, r)
+    finally:
+        for s in sessions:
+            s.close()
