@@ -17,8 +17,9 @@
 
 namespace cgfdm {
 
-// pencil lengths tried (clamped to the grid; the current one is added)
-static const int KCHUNK_CANDIDATES[] = {8, 12, 16, 20, 24, 32, 48, 64, 96, 128, 192, 256};
+// pencil lengths tried (clamped to the grid; the current one is added): the
+// default rule takes 1 to 8
+static const int KCHUNK_CANDIDATES[] = {1, 2, 3, 4, 6, 8, 12, 16, 20, 24, 32, 48, 64, 96, 128, 192, 256};
 
 static int device_sms(int device)
 {
@@ -152,7 +153,7 @@ int Session::autotune(int trial, int *best_kc, int *best_ctas, float *best_ms)
     }
     for (const Cand &c : cand) {
         if (int st = set_tile(c.rows)) return st;
-        if (int st = set_tiling(c.kc, c.ctas)) return st;
+        if (int st = apply_tiling(c.kc, c.ctas)) return st;
         float ms = 0.0f;
         if (int st = tune_load(buf)) return st;
         if (int st = time_steps(1, &ms)) return st;   // first launch of this shape
@@ -163,7 +164,8 @@ int Session::autotune(int trial, int *best_kc, int *best_ctas, float *best_ms)
     }
     if (bms > 0.99f * ms0) bt = t0, bk = k0, bc = c0, bms = ms0;
     if (int st = set_tile(bt)) return st;
-    if (int st = set_tiling(bk, bc)) return st;
+    if (int st = apply_tiling(bk, bc)) return st;
+    if (bk != k0) tiling_chosen_ = true;
     if (int st = tune_load(buf)) return st;
     CU(cudaStreamSynchronize(stream));
     if (best_kc) *best_kc = kchunk_;

@@ -169,7 +169,7 @@ private:
     FaultDev fault_ = {};
     PointDev point_ = {};
     int kchunk_ = 8;
-    bool tiling_chosen_ = false;   // set_tiling was called: batches keep the pencil
+    bool tiling_chosen_ = false;   // by set_tiling or the autotuner: batches keep the pencil
     cudaGraphExec_t graph8_ = nullptr;
     cudaGraph_t graph8_src_ = nullptr;
     cudaEvent_t ev_[4] = {};

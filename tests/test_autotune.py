@@ -101,3 +101,23 @@ def test_batch_autotune_keeps_results(tmp_path):
     finally:
         for s in sessions:
             s.close()
+
+
+@pytest.mark.gpu
+def test_autotuners_reach_the_short_pencils(tmp_path):
+    """On a small grid the default pencil is a plane or two and twice as fast
+    as eight (64 x 60 x 48: 0.11 against 0.22 ms per step), so from a long one
+    the tuners come back to fewer than eight."""
+    c = cases.halfspace_case(NX=64, NY=60, NZ=48, nPML=8, steps=60, n_stations=2)
+    d = cases.write_case(c, str(tmp_path / "run"))
+    with Session(d) as s:
+        assert s.tiling()[0] < 8
+        s.set_tiling(48, 444)
+        assert s.autotune(4)[0] < 8
+    with Session(d) as s, Session(d) as t:
+        for x in (s, t):
+            x.set_tiling(48, 444)          # the batch keeps a chosen pencil
+        with Batch([s, t]) as b:
+            kc, _, _ = b.autotune(4)
+            assert 0 < kc < 8
+        assert s.tiling()[0] == 48
