@@ -23,13 +23,19 @@ from . import Session
 
 def _padded_medium(vp: torch.Tensor, vs: torch.Tensor, rho: torch.Tensor) -> np.ndarray:
     """(Vs, Vp, rho) [nzp][nyp][nxp][3] on the host, the halo filled from the
-    nearest interior point.  Stacked and padded on vp's device, so that one
-    copy brings the finished volume."""
+    nearest interior point.  Interleaved and padded on the host's cores: done on
+    the tensors' device it took 36 B a point there, which torch keeps and the
+    gradient sizes its stores without (144 x 136 x 104: 80 MB).  The interior
+    is copied once and the halo's six slabs after it, x, y, then z."""
     if not vp.shape == vs.shape == rho.shape or vp.dim() != 3:
         raise ValueError("vp, vs and rho must have one shape [nz][ny][nx]")
-    m = torch.stack([t.detach().to(vp.device, torch.float32) for t in (vs, vp, rho)])
-    m = torch.nn.functional.pad(m[None], (3,) * 6, mode="replicate")[0]
-    return m.permute(1, 2, 3, 0).contiguous().cpu().numpy()
+    m = torch.empty(tuple(n + 6 for n in vp.shape) + (3,), dtype=torch.float32, device="cpu")
+    for c, t in enumerate((vs, vp, rho)):
+        m[3:-3, 3:-3, 3:-3, c] = t.detach().to("cpu", torch.float32)
+    m[3:-3, 3:-3, :3], m[3:-3, 3:-3, -3:] = m[3:-3, 3:-3, 3:4], m[3:-3, 3:-3, -4:-3]
+    m[3:-3, :3], m[3:-3, -3:] = m[3:-3, 3:4], m[3:-3, -4:-3]
+    m[:3], m[-3:] = m[3:4], m[-4:-3]
+    return m.numpy()
 
 
 class SeismogramMisfit(torch.autograd.Function):
