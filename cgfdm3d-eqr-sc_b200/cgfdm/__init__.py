@@ -319,7 +319,8 @@ class Session:
     def test_stall(self, item: int, fill: int, wait_cycles: int) -> None:
         """Test hook (cgfdm_test_stall): the next stage launch's work item
         ``item`` leaves plane copy ``fill`` unissued, once, and the stage
-        kernel's bounded waits give up after ``wait_cycles`` clocks."""
+        kernel's bounded waits give up after ``wait_cycles`` clocks.
+        ME-AWENO: tile ``item`` of the next pass along axis ``fill``."""
         self.L.cgfdm_test_stall.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_longlong]
         self._check(self.L.cgfdm_test_stall(self._h, int(item), int(fill), int(wait_cycles)))
 

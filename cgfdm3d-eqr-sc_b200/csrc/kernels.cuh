@@ -206,6 +206,15 @@ struct ScTiling {
 };
 ScTiling sc_tiling(const DevGrid &g);
 
+// Test hook of the passes (stall null in normal runs): while *stall is 1, the
+// CTA that comes to tile `tile` of pass `dir` does not issue its copy and
+// clears *stall, so the wait for it runs out.  wait_limit: clock cycles a
+// bounded wait spins before it gives up (0: 2^31, about a second).
+struct ScStall {
+    int *stall;
+    int dir, tile;
+    long long wait_limit;
+};
 // One launch of a pass: the tensor map of its input with the pass's box (128
 // bytes, from sc_tmap), the tiles in walking order (n0 fastest) and the
 // device error word (bit 0: a bounded wait for a copy gave up, bit 1: the
@@ -215,10 +224,15 @@ struct alignas(64) ScPass {
     ScDirArgs a;
     int n0, n1, n2, total;
     int *err;
+    int *stall;              // ScStall, for this pass
+    int stall_tile;
+    long long wait_limit;
 };
 cudaError_t sc_tmap(void *out, const float *base, const DevGrid &g, int dir);
 cudaError_t launch_sc_dir(int dir, const ScDirArgs &a, const ScTiling &t, const unsigned char *tmap, int *err, int sms,
-                          cudaStream_t st);
+                          const ScStall &stall, cudaStream_t st);
+// tiles of pass dir (0: the build's passes copy nothing ahead)
+int sc_dir_tiles(int dir, const DevGrid &g, const ScTiling &t);
 // Characteristic free surface, halo extrapolation, sponge of the top layers,
 // peak ground velocity and (dis given) the surface-layer displacement, after
 // the third stage of a step.

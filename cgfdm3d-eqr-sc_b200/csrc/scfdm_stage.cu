@@ -479,6 +479,7 @@ __global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const 
     };
     auto issue = [&](int u) {
         int tile, group, rest;
+        if (p.stall && u == p.stall_tile && atomicExch(p.stall, 0) == 1) return;   // test hook
         split(u, tile, group, rest);
         const int m0 = tile * (NPOS - 6) - 2, l0 = CGFDM_HALO + group * NL, r = CGFDM_HALO + rest;
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -493,6 +494,7 @@ __global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const 
         issue(blockIdx.x);                         // the grid has no more CTAs than tiles
     }
     __syncthreads();
+    const long long wlim = p.wait_limit > 0 ? p.wait_limit : (1LL << 31);
     unsigned phase = 0;
 #pragma unroll 1
     for (int u = blockIdx.x; u < p.total; u += gridDim.x, phase ^= 1) {
@@ -516,7 +518,7 @@ __global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const 
         const bool face = have && mi < NPOS - 1 && m >= 2 && m < nd;
         const bool point = have && mi >= 3 && mi <= NPOS - 4 && m < nd;
         // ---- phase A: both WENO states of every position
-        const bool ok = mbar_wait_bounded(bar, phase, 1LL << 31);
+        const bool ok = mbar_wait_bounded(bar, phase, wlim);
         if (ok && have && m >= 2 && m <= nd) {
             // this position's value in the box, the next field SF and the next position SP floats on
             constexpr int SF = DIR == 0 ? 72 * NL : 36 * NL, SP = DIR == 0 ? 1 : NL;
@@ -547,7 +549,7 @@ __global__ void __launch_bounds__(SC_THREADS, SC_TILE_MIN_CTAS) k_sc_tile(const 
             // may still be landing in shared memory when the CTA exits
             if (t == 0) {
                 atomicOr(p.err, 1);
-                if (!mbar_wait_bounded(bar, phase, 1LL << 31)) atomicOr(p.err, 2);
+                if (!mbar_wait_bounded(bar, phase, wlim)) atomicOr(p.err, 2);
             }
             __syncthreads();
             return;
@@ -832,21 +834,34 @@ static cudaError_t launch_pass(ScPass &p, int sms, cudaStream_t st)
 {
     CUDA_TRY(cudaFuncSetAttribute(k_sc_tile<DIR, NPOS, NL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)SC_PASS_SMEM));
-    p.total = p.n0 * p.n1 * p.n2;
     const int grid = std::min(p.total, sms * SC_TILE_MIN_CTAS);
     k_sc_tile<DIR, NPOS, NL><<<grid, SC_THREADS, SC_PASS_SMEM, st>>>(p);
     return cudaGetLastError();
 }
 
+static int lane_groups(int dir, const DevGrid &g, const ScTiling &t)
+{
+    return ((dir == 0 ? g.ny : g.nx) + t.nl[dir] - 1) / t.nl[dir];
+}
+
+int sc_dir_tiles(int dir, const DevGrid &g, const ScTiling &t)
+{
+    return t.ntiles[dir] * lane_groups(dir, g, t) * (dir == 2 ? g.ny : g.nz);
+}
+
 cudaError_t launch_sc_dir(int dir, const ScDirArgs &a, const ScTiling &t, const unsigned char *tmap, int *err, int sms,
-                          cudaStream_t st)
+                          const ScStall &stall, cudaStream_t st)
 {
     const DevGrid &g = a.g;
     ScPass p{};
     std::memcpy(p.tm, tmap, sizeof p.tm);
     p.a = a;
     p.err = err;
-    const int along = t.ntiles[dir], groups = ((dir == 0 ? g.ny : g.nx) + t.nl[dir] - 1) / t.nl[dir];
+    p.stall = stall.dir == dir ? stall.stall : nullptr;
+    p.stall_tile = stall.tile;
+    p.wait_limit = stall.wait_limit;
+    p.total = sc_dir_tiles(dir, g, t);
+    const int along = t.ntiles[dir], groups = lane_groups(dir, g, t);
     if (dir == 0) {
         p.n0 = along, p.n1 = groups, p.n2 = g.nz;
         return launch_pass<0, SCX_NPOS, SCX_NL>(p, sms, st);
@@ -857,8 +872,10 @@ cudaError_t launch_sc_dir(int dir, const ScDirArgs &a, const ScTiling &t, const 
 #else
 cudaError_t sc_tmap(void *, const float *, const DevGrid &, int) { return cudaSuccess; }   // plain loads
 
+int sc_dir_tiles(int, const DevGrid &, const ScTiling &) { return 0; }
+
 cudaError_t launch_sc_dir(int dir, const ScDirArgs &a, const ScTiling &t, const unsigned char *, int *, int,
-                          cudaStream_t st)
+                          const ScStall &, cudaStream_t st)
 {
     const DevGrid &g = a.g;
     if (dir == 0) {

@@ -751,6 +751,7 @@ int Session::launch_step(int step, bool timed_stages)
         float *A = W_[0], *B = W_[1], *C = W_[2];
         const float *win[3] = {A, B, C};
         float *wout[3] = {B, C, A};
+        const ScStall stall{stall_item_ >= 0 ? stall_dev_ : nullptr, stall_fill_, stall_item_, wait_limit_};
         for (int irk = 0; irk < 3; irk++) {
             ScDirArgs a{};
             a.g = g;
@@ -767,7 +768,7 @@ int Session::launch_step(int step, bool timed_stages)
             a.alpha = m.Vp_max;
             if (timed_stages) CU(cudaEventRecord(ev_[2], stream));
             for (int dir = 0; dir < 3; dir++)
-                CU(launch_sc_dir(dir, a, sct_, sc_maps_[irk][dir], err_dev_, sms_, stream));
+                CU(launch_sc_dir(dir, a, sct_, sc_maps_[irk][dir], err_dev_, sms_, stall, stream));
             if (timed_stages) {
                 CU(cudaEventRecord(ev_[3], stream));
                 CU(cudaEventSynchronize(ev_[3]));
@@ -919,14 +920,16 @@ int Session::check_device_error()
 
 int Session::test_stall(int item, int fill, long long wait_cycles)
 {
-    if (m.p.scheme != SCHEME_CGFDM) {
-        err = "the stall hook applies to the CGFDM stage kernel";
+    const bool cg = m.p.scheme == SCHEME_CGFDM;
+    if (!cg && sc_dir_tiles(0, g, sct_) == 0) {
+        err = "the ME-AWENO passes of this build copy nothing ahead";
         return ST_OPTIONS;
     }
     // an item must hold that copy: its planes and the four of its first window
-    if (fill - 3 > kchunk_ && fill - 3 <= m.g.nz)
+    if (cg && fill - 3 > kchunk_ && fill - 3 <= m.g.nz)
         if (int st = apply_tiling(fill - 3, grid_ctas_)) return st;
-    if (item < 0 || item >= stage_items() || fill < 0 || wait_cycles < 0) {
+    if (item < 0 || fill < 0 || wait_cycles < 0 || (!cg && fill > 2) ||
+        item >= (cg ? stage_items() : sc_dir_tiles(fill, g, sct_))) {
         err = "stall hook: item, fill or wait_cycles out of range";
         return ST_ARG;
     }
@@ -935,8 +938,9 @@ int Session::test_stall(int item, int fill, long long wait_cycles)
     CU(cudaMemcpyAsync(stall_dev_, &one, sizeof one, cudaMemcpyHostToDevice, stream));
     CU(cudaStreamSynchronize(stream));
     stall_item_ = item, stall_fill_ = fill, wait_limit_ = wait_cycles;
-    if (int st = build_stage_descs()) return st;
-    // the captured steps hold the old descriptors
+    if (cg)
+        if (int st = build_stage_descs()) return st;
+    // the captured steps hold the old arguments
     if (graph8_) cudaGraphExecDestroy(graph8_);
     if (graph8_src_) cudaGraphDestroy(graph8_src_);
     graph8_ = nullptr;

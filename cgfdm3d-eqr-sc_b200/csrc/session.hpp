@@ -222,6 +222,7 @@ public:
     // Test hook: the next stage launch's work item `item` leaves its plane
     // copy number `fill` unissued, once, and every bounded wait of the stage
     // kernel gives up after `wait_cycles` clocks (0: the default limit).
+    // ME-AWENO: tile `item` of the next pass along axis `fill`.
     int test_stall(int item, int fill, long long wait_cycles);
     // the stage descriptor of RK stage irk (with FP16 storage: for the
     // step-start state of step parity `parity`), and the stage's work items;

@@ -344,12 +344,14 @@ int cgfdm_create_profile(const cgfdm_session *s, double ms[14]);
 
 /* Test hook of the stage kernel's bounded waits.  No counterpart in the
  * reference, whose CHECK macro prints a CUDA error and carries on
- * (src/macro.h:94-103): here every wait of the CGFDM stage kernel for its
- * plane copies is bounded, and a wait that gives up sets a device error word
+ * (src/macro.h:94-103): here every wait of the CGFDM stage kernel and of the
+ * ME-AWENO passes for their copies is bounded, and a wait that gives up sets a device error word
  * that the next cgfdm_run reports as CGFDM_E_TIMEOUT.  After this call the
  * next stage launch's work item `item` leaves its plane copy number `fill`
- * (counted from the item's first plane) unissued, once, and every bounded
- * wait gives up after `wait_cycles` clock cycles (0: the default, 2^31).  The
+ * (counted from the item's first plane) unissued, once -- with ME-AWENO, the
+ * next pass along axis `fill` (0..2) the copy of its tile `item`
+ * (CGFDM_E_OPTIONS in the exact build, whose passes copy nothing ahead) --
+ * and every bounded wait gives up after `wait_cycles` clock cycles (0: the default, 2^31).  The
  * kernel then drains the copies it did issue and returns; the session's
  * state is not usable afterwards, the device is.  For tests only. */
 int cgfdm_test_stall(cgfdm_session *s, int item, int fill, long long wait_cycles);
