@@ -20,6 +20,13 @@ def rel_l2(a: np.ndarray, b: np.ndarray) -> float:
     return float(np.linalg.norm(a - b) / nb)
 
 
+def errors_by_quantity(W, W0, st, st0) -> dict:
+    """rel_l2 of wavefield and station traces, their first three components
+    (velocity, momentum) and the other six (stress, strain) apart."""
+    return {"wavefield 1-3": rel_l2(W[..., :3], W0[..., :3]), "wavefield 4-9": rel_l2(W[..., 3:], W0[..., 3:]),
+            "stations 1-3": rel_l2(st[..., :3], st0[..., :3]), "stations 4-9": rel_l2(st[..., 3:], st0[..., 3:])}
+
+
 def small_halfspace(steps=60, NX=32, NY=32, NZ=24, nPML=6, **kw) -> cases.Case:
     return cases.halfspace_case(NX=NX, NY=NY, NZ=NZ, nPML=nPML, steps=steps, n_stations=6,
                                 depth_m=1000.0, **kw)

@@ -103,10 +103,10 @@ def test_default_build_stays_as_close_to_fp64(tmp_path, nx, ny, nz, nPML, grid, 
             st64, _, W64 = s.run_precise(17, bits=64, wavefield=True)
             s.run(17)
             W, st = s.wavefield(), s.stations()
-        err[flavor] = max(pu.rel_l2(W[..., :3], W64[..., :3]), pu.rel_l2(W[..., 3:], W64[..., 3:]),
-                          pu.rel_l2(st, st64))
-    assert err["exact"] < 1e-5
-    assert err["fast"] <= 2 * err["exact"] + 1e-7
+        err[flavor] = pu.errors_by_quantity(W, W64, st, st64)
+    for q, e in err["exact"].items():
+        assert e < 1e-5, q
+        assert err["fast"][q] <= 2 * e + 1e-7, q
 
 
 @pytest.mark.gpu
