@@ -1155,12 +1155,10 @@ cudaError_t launch_cg_stage_batch_mix(int FB1, int FB2, int FB3, const CgStageDe
 }
 #else
 int cg_stage_ctas_per_sm() { return CG_CTAS_PER_SM; }
-int cg_stage_mix_ctas_per_sm() { return CG_MIX_CTAS_PER_SM; }
-int cg_stage_tile_y() { return TY; }
-size_t cg_stage_smem_bytes(bool mix) { return stage_smem(mix); }
-size_t cg_stage2_smem_bytes() { return stage2_smem(); }
 
 #if CG_TILE_Y == 4
+int cg_stage_mix_ctas_per_sm() { return CG_MIX_CTAS_PER_SM; }
+
 cudaError_t make_field_tmap16(void *out, const __half *base, const DevGrid &gh, int nf)
 {
     const auto encode = tmap_encoder();

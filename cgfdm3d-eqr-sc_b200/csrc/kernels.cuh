@@ -130,9 +130,9 @@ struct alignas(64) CgStageDesc {
     unsigned char tmWc[128];  // split pipeline: the stencil input, interior column box
     CgStageArgs a;
 };
-// The stage kernel's host functions, declared once per tile height: the
-// 32 x 4 build (inline namespace ty4: these names plainly) and the 32 x 8
-// build (cgfdm::ty8, csrc/cgfdm_stage_ty8.cu).
+// The stage kernel's host functions: those of both tile heights, the 32 x 4
+// build (inline namespace ty4: these names plainly) and the 32 x 8 build
+// (cgfdm::ty8, csrc/cgfdm_stage_ty8.cu), and those of 32 x 4 tiles only.
 //
 // launch_cg_stage: one session's stage (ring pipeline), its descriptor passed
 // as a kernel parameter.  launch_cg_stage_batch: session s owns work items
@@ -140,7 +140,7 @@ struct alignas(64) CgStageDesc {
 // memory; all advance with the same FB signs and stage number.
 // launch_cg_stage_split: the split pipeline (the current plane's halo box,
 // interior column boxes for the z window): one session's FP32 stage, a.sweeps
-// 4-row sweeps an item (namespace ty4 only).
+// 4-row sweeps an item.
 // launch_cg_stage_part: the ring pipeline storing into linked parts' halos.
 // launch_cg_stage_mix: mixed-precision storage (the MIX instantiation);
 // launch_cg_stage_batch_mix: the same for a batch of such sessions.
@@ -155,30 +155,26 @@ struct alignas(64) CgStageDesc {
 #define CG_STAGE_FUNCTIONS                                                                                         \
     cudaError_t launch_cg_stage(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,      \
                                 cudaStream_t st);                                                                \
-    cudaError_t launch_cg_stage_part(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas, \
-                                     cudaStream_t st);                                                           \
     cudaError_t launch_cg_stage_batch(int FB1, int FB2, int FB3, int irk, const CgStageDesc *descs,               \
                                       const int *item_start, int nsess, int *work, int grid_ctas,                 \
                                       cudaStream_t st);                                                          \
-    size_t cg_stage_smem_bytes(bool mix = false);                                                               \
-    size_t cg_stage2_smem_bytes();                                                                              \
-    cudaError_t launch_cg_stage_split(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,\
-                                      cudaStream_t st);                                                          \
-    cudaError_t launch_cg_stage_mix(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,  \
-                                    cudaStream_t st);                                                            \
-    cudaError_t launch_cg_stage_batch_mix(int FB1, int FB2, int FB3, const CgStageDesc *descs,                  \
-                                          const int *item_start, int nsess, int *work, int grid_ctas,           \
-                                          cudaStream_t st);                                                      \
-    int cg_stage_mix_ctas_per_sm();                                                                             \
-    cudaError_t make_field_tmap16(void *out, const __half *base, const DevGrid &gh, int nf);                    \
-    cudaError_t launch_impedance_bounds(const float *cjm, DevGrid g, unsigned *out, cudaStream_t st);           \
     cudaError_t make_field_tmap(void *out, const float *base, const DevGrid &g, int nf, bool halo_box,          \
                                 int box_nf = 0);                                                                  \
-    int cg_stage_ctas_per_sm();                                                                                 \
-    int cg_stage_split_ctas_per_sm();                                                                           \
-    int cg_stage_tile_y();
+    int cg_stage_ctas_per_sm();
 inline namespace ty4 {
 CG_STAGE_FUNCTIONS
+cudaError_t launch_cg_stage_split(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,
+                                  cudaStream_t st);
+cudaError_t launch_cg_stage_part(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,
+                                 cudaStream_t st);
+cudaError_t launch_cg_stage_mix(int FB1, int FB2, int FB3, const CgStageDesc &d, int *work, int grid_ctas,
+                                cudaStream_t st);
+cudaError_t launch_cg_stage_batch_mix(int FB1, int FB2, int FB3, const CgStageDesc *descs, const int *item_start,
+                                      int nsess, int *work, int grid_ctas, cudaStream_t st);
+cudaError_t make_field_tmap16(void *out, const __half *base, const DevGrid &gh, int nf);
+cudaError_t launch_impedance_bounds(const float *cjm, DevGrid g, unsigned *out, cudaStream_t st);
+int cg_stage_split_ctas_per_sm();
+int cg_stage_mix_ctas_per_sm();
 }
 namespace ty8 {
 CG_STAGE_FUNCTIONS

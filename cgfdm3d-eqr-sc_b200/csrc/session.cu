@@ -629,7 +629,7 @@ int Session::build_maps()
         for (int b = 0; b < 4; b++) {
             CgStageMaps &M = maps_[eight][b];
             CU(tmap(M.win, W_[b], 9, true));
-            CU(tmap(M.winp, W_[b], 9, false));
+            if (!eight) CU(tmap(M.winp, W_[b], 9, false));   // the split pipeline's sweeps
             CU(tmap(M.cjm, cjm_, 13, false, 3));
             CU(tmap(M.cjm1, cjm_, 13, false, 1));
             CU(tmap(M.wm, W_[0], 9, false));
