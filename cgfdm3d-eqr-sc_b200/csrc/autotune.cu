@@ -18,7 +18,7 @@
 namespace cgfdm {
 
 // pencil lengths tried (clamped to the grid; the current one is added): the
-// default rule takes 1 to 8
+// default rule takes 1 to 12
 static const int KCHUNK_CANDIDATES[] = {1, 2, 3, 4, 6, 8, 12, 16, 20, 24, 32, 48, 64, 96, 128, 192, 256};
 
 static int device_sms(int device)

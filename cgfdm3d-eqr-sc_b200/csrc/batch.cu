@@ -93,7 +93,7 @@ int Batch::create(const std::vector<Session *> &sessions)
             columns += (long long)((x->m.g.nx + 31) / 32) * ((x->m.g.ny + tile_ - 1) / tile_) * x->m.g.nz;
         }
         const int per_sm = mix_ ? cg_stage_mix_ctas_per_sm() : cg_stage_ctas_per_sm();
-        const int k = stage_chunk((columns + nz - 1) / nz, nz, sms * per_sm);
+        const int k = stage_chunk((columns + nz - 1) / nz, nz, sms * per_sm, mix_);
         for (Session *x : s) kchunk_.push_back(x->tiling_chosen() ? x->kchunk() : k);
     }
     BCU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));

@@ -498,7 +498,7 @@ int Session::setup_device()
     nty_ = (G.ny + tile_ - 1) / tile_;
     const long long tiles = (long long)ntx_ * nty_ * (split() ? tile_ / 4 : 1);
     const int ctas = dev_sms * stage_ctas_per_sm();
-    kchunk_ = stage_chunk(tiles, G.nz, ctas);
+    kchunk_ = stage_chunk(tiles, G.nz, ctas, mix_);
     nchunk_ = (G.nz + kchunk_ - 1) / kchunk_;
     grid_ctas_ = (int)std::min<long long>(ctas, tiles * nchunk_);
 
@@ -524,22 +524,37 @@ int Session::setup_device()
 }
 
 // Planes per work item of the persistent stage launch, for `tiles` column
-// tiles of nz planes on `ctas` resident CTAs.  An item costs its planes and
-// about 0.7 of one more (its first window has to arrive before it can
-// start), and a launch its items' share a CTA and about one item more (the
-// first CTAs start together and the last ones end alone), so short items win
-// where there are few of them and long ones where there are many.  Beyond 8
-// planes neighbouring tiles drift apart in z and stop sharing halo planes
-// through L2.  Measured, ms per step on 32 x 4 tiles with 1, 2, 3, 5, 8, 12
-// planes: 64x60x48 0.118 0.132 0.133 0.155 0.215 0.271, 128x128x96 0.573
-// 0.527 0.523 0.541 0.602 0.685, 213x151x117 1.24 1.08 1.04 1.01 1.04 1.11.
-int stage_chunk(long long tiles, int nz, int ctas)
+// tiles of nz planes on `ctas` resident CTAs.  An item costs its planes and a
+// window (its first planes have to arrive, and with FP16 storage to be
+// converted, before it can start: 0.7 and 2 of a plane's time, from one plane
+// an item against twelve on 400x400x200), and a launch its items' share a CTA
+// and about one item more (the first CTAs start together and the last ones end
+// alone), so short items win where there are few of them and long ones where
+// there are many.  At 8 planes (FP16 12) the gain of longer ones is gone.
+// Measured, ms per step with 1, 2, 3, 4, 5, 6, 8, 12 planes, the rule's in
+// brackets (FP32 split pipeline, 32 x 8 items; the ring pipeline is alike):
+//   64x60x48     0.116 [0.117] 0.135 0.122 0.135 0.146 0.180 0.239
+//   90x80x64     0.228 [0.211] 0.204 0.221 0.217 0.238 0.253 0.290
+//   128x128x96   0.578 0.507 0.480 [0.471] 0.465 0.478 0.499 0.563
+//   160x152x100  0.832 0.716 0.652 0.645 [0.639] 0.636 0.658 0.720
+//   213x151x117  1.286 1.074 0.993 0.954 0.924 0.926 [7 planes] 0.916 0.962
+//   400x400x200  9.40 7.37 6.68 6.37 6.13 6.02 [5.84] 5.85
+// and with FP16 storage:
+//   64x60x48     0.227 0.206 [0.201] 0.221 0.204 0.186 0.214 0.277
+//   90x80x64     0.492 0.389 0.350 0.354 [0.335] 0.344 0.357 0.417
+//   128x128x96   1.34 0.978 0.871 0.803 0.756 0.751 [0.744] 0.769
+//   213x151x117  3.22 2.25 1.94 1.73 1.63 1.57 1.51 [9 planes] 1.46
+//   400x400x200  24.9 16.6 13.6 12.0 11.1 10.6 9.97 [9.35]
+// so the rule stays within 4 % of the best (8 % on the smallest FP16 grid).
+int stage_chunk(long long tiles, int nz, int ctas, bool mix)
 {
+    const int most = mix ? 12 : 8;
+    const double window = mix ? 2.0 : 0.7;
     int best = 1;
     double least = 0.0;
-    for (int k = 1; k <= std::min(8, nz); k++) {
+    for (int k = 1; k <= std::min(most, nz); k++) {
         const double items = (double)tiles * ((nz + k - 1) / k);
-        const double t = (items / ctas + 1.0) * (k + 0.7);
+        const double t = (items / ctas + 1.0) * (k + window);
         if (k == 1 || t < least) best = k, least = t;
     }
     const int n = (nz + best - 1) / best;

@@ -32,7 +32,7 @@ constexpr int STAGE_IN[4] = {0, 1, 2, 3}, STAGE_OUT[4] = {1, 2, 3, 0};
 #endif
 
 // planes per work item of a stage launch (csrc/session.cu)
-int stage_chunk(long long tiles, int nz, int ctas);
+int stage_chunk(long long tiles, int nz, int ctas, bool mix);
 
 // How a batch's launch cuts a session's grid: rows of the column tiles (4 or
 // 8) and planes per work item.  The batch's own: the sessions keep theirs.

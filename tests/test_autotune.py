@@ -105,9 +105,9 @@ def test_batch_autotune_keeps_results(tmp_path):
 
 @pytest.mark.gpu
 def test_autotuners_reach_the_short_pencils(tmp_path):
-    """On a small grid the default pencil is a plane or two and twice as fast
-    as eight (64 x 60 x 48: 0.11 against 0.22 ms per step), so from a long one
-    the tuners come back to fewer than eight."""
+    """On a small grid the default pencil is a plane or two and much faster than
+    eight (64 x 60 x 48: 0.12 against 0.18 ms per step), so from a long one the
+    tuners come back to fewer than eight."""
     c = cases.halfspace_case(NX=64, NY=60, NZ=48, nPML=8, steps=60, n_stations=2)
     d = cases.write_case(c, str(tmp_path / "run"))
     with Session(d) as s:
