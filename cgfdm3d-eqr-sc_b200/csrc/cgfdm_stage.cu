@@ -24,12 +24,11 @@
 // fixed shared-memory offset.  Metric, medium and RK inputs are plain
 // coalesced loads issued before the ring wait.
 //
-// What bounds it: 400 x 400 x 200, the default build, moves 24 GB a step in
-// 6.35 ms (3.8 TB/s of algorithmic bytes; DRAM at 60 % of its nominal peak in
-// the middle stages, issue slots 45-50 % full, the rest waits for memory with
-// twelve warps an SM).  Before the zero metric terms, the factored sums and
-// the running sum's going it was 8.2 ms, 1174-1304 instructions a warp of
-// points against 830-960 now.
+// What bounds it: 400 x 400 x 200, the default build, moves 21.8 GB a step in
+// 6.4 ms (3.4 TB/s of algorithmic bytes; DRAM at 37-56 % of its peak, issue
+// slots 45-48 % full, the rest waits for memory with twelve warps an SM).
+// Before the zero metric terms, the factored sums and the running sum's going
+// it was 8.2 ms, 1174-1304 instructions a warp of points against 720-970 now.
 //
 // Every wait on an mbarrier is bounded: on timeout the CTA records the fact
 // in a device error word, waits (bounded) for its copies in flight and exits.
